@@ -62,6 +62,41 @@ def test_mla_prefill_and_mixed():
     _case([1, 37, 3, 64], [50, 0, 700, 20], 16, 512, 64)
 
 
+# tiles of 128 (token, head) rows, chunks of 128 keys in pages of 16: one row, rows across tokens, tiles that end inside a
+# request, contexts around a page and a chunk, several items per pair of SMs, requests without tokens
+@pytest.mark.parametrize("q_lens,ctx,H", [([1], [0], 1), ([1, 1, 1], [15, 16, 17], 3), ([1, 1, 1, 1], [126, 127, 128, 129], 128),
+                                          ([45, 0, 130, 1], [0, 64, 200, 3000], 24), ([300], [33], 128)])
+def test_mla_tiles_of_128_rows(q_lens, ctx, H):
+    _case(q_lens, ctx, H, 512, 64)
+
+
+def test_mla_rows_of_the_cache_that_nothing_wrote_do_not_matter():
+    from vllm_torchtpu_b200.ops import cuda
+    g = torch.Generator(device=DEV).manual_seed(3)
+    seq, H = [70, 131, 16], 16
+    cache = torch.full((24, 16, 576), float("nan"), dtype=torch.bfloat16, device=DEV)
+    bt = torch.zeros(3, 12, dtype=torch.int32, device=DEV)
+    at = 1
+    for r, s in enumerate(seq):
+        n = -(-s // 16)
+        bt[r, :n] = torch.arange(at, at + n, device=DEV)
+        rows = cache[at:at + n].view(-1, 576)
+        rows[:s] = torch.randn(s, 576, device=DEV, generator=g).bfloat16()
+        at += n
+    # one request decodes, one has a chunk; two rows of padding behind the step's tokens
+    lens = [1, 40, 16]
+    qsl = torch.tensor([0, 1, 41, 57], dtype=torch.int32, device=DEV)
+    q = torch.randn(59, H, 576, device=DEV, generator=g).bfloat16()
+    sl = torch.tensor(seq, dtype=torch.int32, device=DEV)
+    meta = AttentionMetadata(None, None, bt, sl, qsl, 3, 57, num_decode_reqs=1, max_query_len=40, max_seq_len=131,
+                             padded_num_reqs=3, padded_num_tokens=59)
+    out, lse = cuda.mla_paged_attention(q, cache, meta, 576 ** -0.5, 512, return_lse=True)
+    want = ref.mla_paged_attention(q[:57], torch.nan_to_num(cache), bt, sl, qsl, 576 ** -0.5, 512, num_reqs=3)
+    torch.testing.assert_close(out[:57].float(), want.float(), rtol=2e-2, atol=2e-2)
+    assert out[57:].eq(0).all() and torch.isneginf(lse[57:]).all()
+    assert sum(lens) == 57 and cuda.check_status() == 0
+
+
 def test_mla_sparse_topk():
     _case([1, 5, 1], [400, 90, 7], 32, 512, 64, topk=64)
 

@@ -22,7 +22,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relax
 
 
 CHECKED_LIB_NAME = "libb200_attention_checked.so"
-CHECKED_SOURCES = ("attention.cu", "attention_tc.cu", "attention_mla.cu")
+CHECKED_SOURCES = ("attention.cu", "attention_tc.cu", "attention_mla.cu", "attention_mla_tc.cu")
 
 
 def lib_path() -> str:
@@ -73,7 +73,7 @@ def _headers_mtime() -> float:
 
 # sources whose kernels a model family launches on one GPU (families not listed need the full library)
 FAMILY_SOURCES = {
-    "mazivik": ("attention_mla.cu", "elementwise.cu", "gemm_2sm_tcgen05.cu", "gemm_simt.cu", "gemm_tcgen05.cu",
+    "mazivik": ("attention_mla.cu", "attention_mla_tc.cu", "elementwise.cu", "gemm_2sm_tcgen05.cu", "gemm_simt.cu", "gemm_tcgen05.cu",
                 "layer_norm.cu", "runtime.cu", "sample.cu"),
     "popanex": ("attention.cu", "attention_simt.cu", "attention_tc.cu", "elementwise.cu", "gemm_2sm_tcgen05.cu",
                 "gemm_simt.cu", "gemm_tcgen05.cu", "layer_norm.cu", "linear_attention.cu", "norm_cache.cu", "runtime.cu",

@@ -1239,6 +1239,26 @@ extern "C" int b200_make_tmap_3d_bf16(void* out_map, const void* ptr, uint64_t d
   return 0;
 }
 
+extern "C" int b200_make_tmap_4d_bf16(void* out_map, const void* ptr, const uint64_t dims[4], const uint64_t stride_bytes[3],
+                                      const uint32_t box[4]) {
+  auto fn = b200::get_encode_fn();
+  if (!fn) {
+    b200_set_last_error("cuTensorMapEncodeTiled not available", __FILE__, __LINE__);
+    return -1;
+  }
+  const cuuint64_t gdim[4] = {dims[0], dims[1], dims[2], dims[3]};
+  const cuuint64_t gstride[3] = {stride_bytes[0], stride_bytes[1], stride_bytes[2]};
+  const cuuint32_t b[4] = {box[0], box[1], box[2], box[3]}, estr[4] = {1, 1, 1, 1};
+  const CUresult r = fn(reinterpret_cast<CUtensorMap*>(out_map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr),
+                        gdim, gstride, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    b200_set_last_error("cuTensorMapEncodeTiled (4D) failed", __FILE__, __LINE__);
+    return (int)r;
+  }
+  return 0;
+}
+
 namespace b200 {
 
 struct TmapKey {

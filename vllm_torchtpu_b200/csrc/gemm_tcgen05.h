@@ -27,6 +27,8 @@ int b200_make_tmap_2d_bytes_linear(void* out_map, const void* ptr, uint64_t rows
 int b200_make_tmap_3d_bf16(void* out_map, const void* ptr, uint64_t dx, uint64_t dy, uint64_t dz,
                            uint64_t stride_y_bytes, uint64_t stride_z_bytes, uint32_t bx, uint32_t by,
                            uint32_t bz);
+int b200_make_tmap_4d_bf16(void* out_map, const void* ptr, const uint64_t dims[4], const uint64_t stride_bytes[3],
+                           const uint32_t box[4]);
 
 #ifdef __cplusplus
 }

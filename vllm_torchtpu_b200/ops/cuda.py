@@ -41,7 +41,7 @@ def bad_index_count() -> int:
     by the bounds-checked library, ``B200_BOUNDS_CHECK=1``)."""
     total = 0
     for name in ("b200_bad_index_count_attention", "b200_bad_index_count_attention_tc",
-                 "b200_bad_index_count_attention_mla"):
+                 "b200_bad_index_count_attention_mla", "b200_bad_index_count_attention_mla_tc"):
         v = ctypes.c_uint(0)
         _check(getattr(lib(), name)(ctypes.byref(v)), name)
         total += v.value

@@ -22,6 +22,32 @@ def mla_write_cache(cache, kv_c, k_pe, slot_mapping):
     count_launch()
 
 
+def _mla_tc(q, cache, meta, scale, R, return_lse):
+    """The two-SM kernel: rows of 512 + 64 values."""
+    T, H, _ = q.shape
+    nb, bs, _ = cache.shape
+    ws = _c.Workspace.get(q.device)
+    out = torch.empty((T, H, 512), dtype=q.dtype, device=q.device)
+    lse = torch.empty((T, H), dtype=torch.float32, device=q.device) if return_lse else None
+    # split-KV when the tiles of 128 rows are fewer than the pairs of SMs.  Inside a captured graph the choice depends on the
+    # batch shape only (lengths change between replays; a split without keys contributes lse = -inf).
+    tiles = max(R, T * H // 128)
+    splits = max(1, min(16, _c._sms // max(1, tiles)))
+    if splits > 1 and not torch.cuda.is_current_stream_capturing():
+        splits = max(1, min(splits, int(meta.max_seq_len or 0) // 128))
+    part = part_lse = None
+    if splits > 1:
+        part = torch.empty((splits, T, H, 512), dtype=torch.float32, device=q.device)
+        part_lse = torch.empty((splits, T, H), dtype=torch.float32, device=q.device)
+    _c._check(_c.lib().b200_mla_attention_tc(
+        _c._p(q), _c._p(cache), _c._p(out), _c._p(lse), _c._p(meta.block_tables), _c._p(meta.seq_lens),
+        _c._p(meta.query_start_loc), c_int(T), c_int(R), c_int(H), c_int(meta.block_tables.shape[1]), c_int(bs),
+        c_longlong(nb), c_float(scale), c_int(splits), _c._p(part), _c._p(part_lse), _c._p(ws.status), c_int(_c._sms),
+        _c._stream()), "mla_attention_tc")
+    count_launch(2 if splits > 1 else 1)
+    return (out, lse) if return_lse else out
+
+
 def mla_paged_attention(q_latent, cache, meta, scale, kv_lora_rank: int, *, topk_indices=None,
                         return_lse: bool = False):
     """Absorbed-query MLA over the paged latent cache; dense, or sparse when ``topk_indices`` [T, K] is given."""
@@ -43,6 +69,8 @@ def mla_paged_attention(q_latent, cache, meta, scale, kv_lora_rank: int, *, topk
             "mla_attention_simt")
         count_launch()
         return out
+    if topk_indices is None and Dq == 576 and kv_lora_rank == 512 and bs % 16 == 0 and not (q.data_ptr() | cache.data_ptr()) & 15:
+        return _mla_tc(q, cache, meta, scale, R, return_lse)
     # prefill of a head count that leaves MMA rows empty: tiles over the (token, head) rows of every request
     flat = 0
     if H % 16 and topk_indices is None and meta.query_start_loc_cpu is not None and meta.max_query_len > 1:
