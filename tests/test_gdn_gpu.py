@@ -60,3 +60,72 @@ def test_kda_forward_two_steps(Hk, Hv, dk, dv, lb):
         err = (got.float() - want.float()).abs().max().item()
         assert err <= 3e-2 * want.float().abs().max().item() + 1e-2, err
     torch.testing.assert_close(pools[0], pools[1], rtol=3e-2, atol=3e-2)
+
+
+# chunks of the convolution (32 tokens) and of the staged tokens (16 and 8), portions shorter than the carried window, requests
+# without tokens or without a state, rows behind the step's tokens, value widths that are no multiple of the 64 columns of a
+# CTA or of a vector, more requests than a warp has lanes
+@pytest.mark.parametrize("Hk,Hv,dk,dv", [(1, 2, 128, 128), (1, 1, 64, 72), (2, 2, 32, 33)])
+@pytest.mark.parametrize("q_lens,ctx", [([1, 2, 3, 31, 32, 33, 0, 65], [0, 1, 2, 9, 0, 70, 5, 0]), ([1] * 35, [0, 4, 9, 30, 2] * 7)])
+def test_ragged_portions_and_untouched_rows(Hk, Hv, dk, dv, q_lens, ctx):
+    from vllm_torchtpu_b200.ops import cuda
+    gen = torch.Generator(device=DEV).manual_seed(7)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)                      # noqa: E731
+    C, R, T = 2 * Hk * dk + Hv * dv, len(q_lens), sum(q_lens)
+    slots = [(3 * r + 1) % (R + 2) if (R + 2) % 3 else r for r in range(R)]
+    off = 4 if R > 4 else None
+    if off is not None:
+        slots[off] = -1                                                               # no state: rows of zeros
+    meta = _meta(q_lens, ctx, slots)
+    pad = 3
+    mixed, conv_w = rnd(T + pad, C).bfloat16(), (rnd(C, 4) * 0.3).bfloat16()
+    a, b, ac = rnd(T + pad, Hv).bfloat16(), rnd(T + pad, Hv).bfloat16(), rnd(T + pad, Hv, dk).bfloat16()
+    A_log, dt, dtc = rnd(Hv) * 0.3, rnd(Hv) * 0.3, rnd(Hv, dk) * 0.3
+    conv, rec = rnd(R + 2, C, 3).bfloat16(), rnd(R + 2, Hv, dk, dv) * 0.1
+    got_pools, want_pools = [conv.clone(), rec.clone()], [conv.clone(), rec.clone()]
+    got = cuda.gdn_forward(mixed, a, b, meta, *got_pools, conv_w, A_log, dt, Hk, Hv, dk, dv)
+    keep = [r for r in range(R) if slots[r] >= 0]
+    rows = torch.cat([torch.arange(sum(q_lens[:r]), sum(q_lens[:r + 1]), device=DEV) for r in keep])
+    sub = _meta([q_lens[r] for r in keep], [ctx[r] for r in keep], [slots[r] for r in keep])
+    want = g.gdn_forward(mixed[rows], a[rows], b[rows], None, sub, *want_pools, conv_w, A_log, dt, Hk, Hv, dk, dv)
+
+    def close(x, y):
+        # convolved values are bf16 on both sides: a value that rounds the other way moves a result by 2^-8 of it
+        assert (x.float() - y.float()).abs().max() <= 2e-2 * y.float().abs().max() + 1e-3
+    rest = torch.ones(T + pad, dtype=torch.bool, device=DEV)
+    rest[rows] = False
+    close(got[rows], want)
+    assert got[rest].eq(0).all()
+    assert torch.equal(got_pools[0], want_pools[0])
+    close(got_pools[1], want_pools[1])
+    y = cuda.short_conv(mixed, meta, conv.clone(), conv_w)
+    assert y[rest].eq(0).all()
+    q, k, v = y.split([Hk * dk, Hk * dk, Hv * dv], -1)
+    q, k, v = q.reshape(-1, Hk, dk), k.reshape(-1, Hk, dk), v.reshape(-1, Hv, dv)
+    got_rec, want_rec = rec.clone(), rec.clone()
+    got = cuda.kda_forward(q, k, v, ac, b, meta, got_rec, A_log, dtc)
+    want = g.kda_forward(q[rows], k[rows], v[rows], ac[rows], b[rows], sub, want_rec, A_log, dtc)
+    close(got[rows], want)
+    assert got[rest].eq(0).all()
+    close(got_rec, want_rec)
+
+
+def test_decays_that_underflow():
+    """A decay of exactly zero forgets the state; products of decays leave the range of fp32 within a few tokens."""
+    from vllm_torchtpu_b200.ops import cuda
+    gen = torch.Generator(device=DEV).manual_seed(8)
+    Hk, Hv, dk, dv, T = 1, 1, 128, 128, 200
+    C = 2 * Hk * dk + Hv * dv
+    mixed = torch.randn(T, C, device=DEV, generator=gen).bfloat16()
+    a = torch.full((T, Hv), 60.0, device=DEV).bfloat16()                 # g = -60 e: below exp's range
+    a[::3] = -3.0
+    a[100:] = 3.0
+    b = torch.randn(T, Hv, device=DEV, generator=gen).bfloat16()
+    conv_w = (torch.randn(C, 4, device=DEV, generator=gen) * 0.3).bfloat16()
+    A_log, dt = torch.ones(Hv, device=DEV), torch.zeros(Hv, device=DEV)
+    pools = [(torch.zeros(1, C, 3, device=DEV, dtype=torch.bfloat16), torch.ones(1, Hv, dk, dv, device=DEV)) for _ in range(2)]
+    meta = _meta([T], [5], [0])
+    got = cuda.gdn_forward(mixed, a, b, meta, *pools[0], conv_w, A_log, dt, Hk, Hv, dk, dv)
+    want = g.gdn_forward(mixed, a, b, None, meta, *pools[1], conv_w, A_log, dt, Hk, Hv, dk, dv)
+    assert (got.float() - want.float()).abs().max() <= 2e-2 * want.float().abs().max()
+    assert (pools[0][1] - pools[1][1]).abs().max() <= 2e-2 * pools[1][1].abs().max()
