@@ -62,11 +62,12 @@ def test_kda_forward_two_steps(Hk, Hv, dk, dv, lb):
     torch.testing.assert_close(pools[0], pools[1], rtol=3e-2, atol=3e-2)
 
 
-# chunks of the convolution (32 tokens) and of the staged tokens (16 and 8), portions shorter than the carried window, requests
+# chunks of the convolution (32 tokens), of the rule on the tensor cores (64) and of the staged tokens (16 and 8), portions shorter than the carried window, requests
 # without tokens or without a state, rows behind the step's tokens, value widths that are no multiple of the 64 columns of a
 # CTA or of a vector, more requests than a warp has lanes
 @pytest.mark.parametrize("Hk,Hv,dk,dv", [(1, 2, 128, 128), (1, 1, 64, 72), (2, 2, 32, 33)])
-@pytest.mark.parametrize("q_lens,ctx", [([1, 2, 3, 31, 32, 33, 0, 65], [0, 1, 2, 9, 0, 70, 5, 0]), ([1] * 35, [0, 4, 9, 30, 2] * 7)])
+@pytest.mark.parametrize("q_lens,ctx", [([1, 2, 3, 31, 32, 33, 0, 65], [0, 1, 2, 9, 0, 70, 5, 0]), ([1] * 35, [0, 4, 9, 30, 2] * 7),
+                                        ([64, 128, 129, 2, 1, 200, 63], [0, 3, 0, 8, 8, 64, 1]), ([3, 2, 5, 1], [0, 1, 4, 2])])
 def test_ragged_portions_and_untouched_rows(Hk, Hv, dk, dv, q_lens, ctx):
     from vllm_torchtpu_b200.ops import cuda
     gen = torch.Generator(device=DEV).manual_seed(7)

@@ -646,13 +646,19 @@ static int launch_step(StepParams p, int dk, int dv, cudaStream_t stream) {
 
 using namespace b200;
 
+extern "C" int b200_gdn_chunks(const void* y, int Cy, const void* a, const void* b, int lda, const float* A_log,
+                               const float* dt_bias, float* rec_pool, void* out, float* scratch, const int* qsl,
+                               const int* seq_lens, const int* slots, int R, int T, int Hk, int Hv, int* status,
+                               cudaStream_t stream);
+
 // mixed [T, C] (C = 2*Hk*dk + Hv*dv, row stride ldx), a/b [T, Hv] (row stride lda).
-// scratch: conv_out [T, C] bf16, qn/kn [T, Hk, dk] fp32, g/beta [T, Hv] fp32 (caller allocates).
+// scratch of the caller: conv_out [T, C] bf16; qn/kn [T, Hk, dk] fp32 and g/beta [T, Hv] fp32, or (heads of 128 / 128) the
+// chunks' (gdn_chunk.cu), which selects that path.  With heads of 128 / 128 and T <= R none is used.
 extern "C" int b200_gdn_forward(const void* mixed, int ldx, const void* a, const void* b, int lda,
                                 const void* conv_w, const float* A_log, const float* dt_bias, void* conv_pool,
                                 float* rec_pool, void* conv_out, float* qn, float* kn, float* g, float* beta,
-                                void* out, const int* qsl, const int* seq_lens, const int* slots, int R, int T,
-                                int Hk, int Hv, int dk, int dv, int conv_k, cudaStream_t stream) {
+                                float* chunks, void* out, const int* qsl, const int* seq_lens, const int* slots, int R, int T,
+                                int Hk, int Hv, int dk, int dv, int conv_k, int* status, cudaStream_t stream) {
   if (R <= 0 || T <= 0) return 0;
   const int C = 2 * Hk * dk + Hv * dv;
   if (conv_k != 4 || dv * (dk / 32) > 512 || (dk != 128 && dk != 64 && dk != 32)) {
@@ -668,8 +674,15 @@ extern "C" int b200_gdn_forward(const void* mixed, int ldx, const void* a, const
   int rc = launch_step<false>(sp, dk, dv, stream);
   if (rc <= 0) return rc;
   const int skip = dk == 128 && dv == 128 && R <= 65535 && !((uintptr_t)conv_w & 7);
+  if (conv_out == nullptr || (chunks != nullptr ? !skip : (qn == nullptr || kn == nullptr || g == nullptr || beta == nullptr))) {
+    b200_set_last_error("gdn_forward: scratch is missing", __FILE__, __LINE__);
+    return -1;
+  }
   rc = launch_conv(mixed, conv_out, conv_pool, conv_w, qsl, seq_lens, slots, R, T, C, ldx, skip, stream);
   if (rc) return rc;
+  if (chunks != nullptr)
+    return b200_gdn_chunks(conv_out, C, a, b, lda, A_log, dt_bias, rec_pool, out, chunks, qsl, seq_lens, slots, R, T, Hk, Hv,
+                           status, stream);
   const int work = T * (Hk * 32 > Hv ? Hk * 32 : Hv);
   B200_CUDA_CHECK(launch_pdl(gdn_prep_kernel, dim3((work + 255) / 256), dim3(256), (size_t)0, stream,
                              (const __nv_bfloat16*)conv_out, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, A_log, dt_bias,

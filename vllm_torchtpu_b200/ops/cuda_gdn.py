@@ -9,25 +9,37 @@ from . import count_launch
 from . import cuda as _c
 
 
+CHUNK_WORDS = 128 * 64 + 4 * 64           # scratch of a (chunk, head) in gdn_chunk.cu
+
+
 def gdn_forward(mixed, a, b, meta, conv_pool, rec_pool, conv_w, A_log, dt_bias, Hk, Hv, dk, dv):
     """mixed [T, 2*Hk*dk + Hv*dv] bf16 (may be a column slice), a/b [T, Hv] -> o [T, Hv, dv]."""
     _c._require_bf16(mixed, a, b, conv_w)
     T, C = mixed.shape
     dev = mixed.device
     R = meta.padded_num_reqs if meta.padded_num_reqs is not None else meta.num_reqs
-    conv_out = torch.empty((T, C), dtype=torch.bfloat16, device=dev)
-    qn = torch.empty((T, Hk, dk), dtype=torch.float32, device=dev)
-    kn = torch.empty_like(qn)
-    g = torch.empty((T, Hv), dtype=torch.float32, device=dev)
-    beta = torch.empty_like(g)
-    out = torch.empty((T, Hv, dv), dtype=torch.bfloat16, device=dev)
+    def new(*shape, dtype=torch.float32):
+        return torch.empty(shape, dtype=dtype, device=dev)
+    out = new(T, Hv, dv, dtype=torch.bfloat16)
+    conv_out = qn = kn = g = beta = chunks = None
+    step = dk == dv == 128 and conv_w.data_ptr() % 8 == 0           # single tokens have their own kernel
+    if not step or T > R:
+        conv_out = new(T, C, dtype=torch.bfloat16)
+        # Chunks of 64 tokens on the tensor cores, or token by token: a token costs about 0.7 us there, a request's chunk
+        # about 8 us with the work in front of it.  A wrong length costs time only.  (Scratch of at most 1 GB: 0.5 KB a token and head.)
+        longest = meta.max_query_len if meta.max_query_len > 1 else T - R + 1
+        words = (T // 64 + R) * Hv * CHUNK_WORDS
+        if step and longest > 16 and words <= 1 << 28:
+            chunks = new(words)
+        else:
+            qn, kn, g, beta = new(T, Hk, dk), new(T, Hk, dk), new(T, Hv), new(T, Hv)
     _c._check(_c.lib().b200_gdn_forward(
         _c._p(mixed), c_int(mixed.stride(0)), _c._p(a), _c._p(b), c_int(a.stride(0)), _c._p(conv_w),
         _c._p(A_log), _c._p(dt_bias), _c._p(conv_pool), _c._p(rec_pool), _c._p(conv_out), _c._p(qn), _c._p(kn),
-        _c._p(g), _c._p(beta), _c._p(out), _c._p(meta.query_start_loc), _c._p(meta.seq_lens),
+        _c._p(g), _c._p(beta), _c._p(chunks), _c._p(out), _c._p(meta.query_start_loc), _c._p(meta.seq_lens),
         _c._p(meta.state_slots), c_int(R), c_int(T), c_int(Hk), c_int(Hv), c_int(dk), c_int(dv),
-        c_int(conv_w.shape[1]), _c._stream()), "gdn_forward")
-    count_launch(3)
+        c_int(conv_w.shape[1]), _c._p(_c.Workspace.get(dev).status), _c._stream()), "gdn_forward")
+    count_launch((4 if step else 3) if conv_out is not None else 1)
     return out
 
 
