@@ -188,6 +188,42 @@ def test_sampling_cluster_kernel_on_an_odd_vocabulary():
     assert torch.equal(got.long(), want)
 
 
+# keys per thread of the cluster kernel (8, 32, 40, 64) at their limits, the single-CTA kernel on both sides of them; lists that
+# overflow (equal logits), fewer finite logits than k, k at the limit of the list
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [4095, 4096, 32768, 32770, 131072, 151936, 163841, 262145])
+def test_sampling_sizes_and_types(V, dtype):
+    R = 12
+    g = torch.Generator(device=DEV).manual_seed(V)
+    logits = (torch.randn(R, V, device=DEV, generator=g) * 2.0).to(dtype)
+    logits[0] = 0.5
+    logits[1, 7:] = -float("inf")
+    logits[2, ::2] = -float("inf")
+    logits[3] *= 100.0
+    temp = torch.rand(R, device=DEV, generator=g) + 0.3
+    temp[11] = 0.0
+    top_k = torch.tensor([50, 50, 512, 511, 1, 0, 0, 20, 600, 2, 3000, 5], device=DEV, dtype=torch.int32)
+    top_p = torch.tensor([0.9, 0.9, 0.5, 1.0, 1.0, 0.95, 1.0, 0.3, 0.9, 0.99, 0.8, 1.0], device=DEV)
+    u = cu().philox_uniform(R, V, 5, 2, DEV)
+    got = cu().sample(logits, temp, top_k, top_p, uniform=u)
+    # the statement with ties at a threshold kept (bf16 logits tie): masses in 64 bits
+    x = logits.float() * (1.0 / temp.clamp_min(1e-5))[:, None]
+    want = logits.float().argmax(-1)
+    for r in range(R - 1):
+        s = x[r].sort(descending=True).values
+        k = int(top_k[r])
+        kept = x[r] >= (s[k - 1] if 0 < k < V else s[-1])
+        if top_p[r] < 1:
+            mass = torch.exp(x[r].double() - s[0].double()) * kept
+            order = x[r].argsort(descending=True)
+            # the first value at which the mass from the top on, ties included, reaches its share
+            at = int((mass[order].cumsum(0) >= top_p[r].double() * mass.sum()).nonzero()[0])
+            kept &= x[r] >= x[r][order[at]]
+        noisy = x[r] - torch.log(-torch.log(u[r].clamp(1e-20, 1.0 - 1e-7)))
+        want[r] = noisy.masked_fill(~kept, float("-inf")).argmax()
+    assert torch.equal(got.long(), want)
+
+
 def test_logprobs():
     R, V = 5, 32000
     logits = torch.randn(R, V, device=DEV).bfloat16()

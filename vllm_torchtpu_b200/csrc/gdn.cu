@@ -23,15 +23,18 @@ struct Row<1> {
   __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *p; }
   __device__ __forceinline__ void store(__nv_bfloat16* p) const { *p = v; }
   __device__ __forceinline__ float get(int) const { return __bfloat162float(v); }
-  __device__ __forceinline__ void set(int, float f) { v = __float2bfloat16(f); }
+  __device__ __forceinline__ void set(const float (&f)[1]) { v = __float2bfloat16(f[0]); }
 };
 template <>
 struct Row<8> {
-  __nv_bfloat16 v[8];
+  __align__(16) __nv_bfloat16 v[8];
   __device__ __forceinline__ void load(const __nv_bfloat16* p) { *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(p); }
   __device__ __forceinline__ void store(__nv_bfloat16* p) const { *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(v); }
   __device__ __forceinline__ float get(int i) const { return __bfloat162float(v[i]); }
-  __device__ __forceinline__ void set(int i, float f) { v[i] = __float2bfloat16(f); }
+  __device__ __forceinline__ void set(const float (&f)[8]) {      // (two conversions at a time)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) reinterpret_cast<__nv_bfloat162*>(v)[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  }
 };
 
 // x [T, C] bf16 -> y [T, C] bf16 (convolution of 4 taps, then SiLU).  grid (ceil(C / (128 VEC)), T / 32 + R): a CTA takes up
@@ -67,8 +70,8 @@ gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__
   }
   if (c >= C) return;
   Row<VEC> zero;
-#pragma unroll
-  for (int e = 0; e < VEC; ++e) zero.set(e, 0.f);
+  const float nothing[VEC] = {};
+  zero.set(nothing);
   for (int t = max(0, qsl[R]) + blockIdx.y; t < T; t += gridDim.y) zero.store(y + (size_t)t * C + c);
   if (r < 0) return;
   const int qs = qsl[r], len = qsl[r + 1] - qs, t0 = chunk * CONV_ROWS, t1 = min(len, t0 + CONV_ROWS);
@@ -148,7 +151,7 @@ gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
       if (t + i >= t1) break;
-      Row<VEC> out;
+      float o[VEC];
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
         const float v = in[i].get(e);
@@ -156,11 +159,13 @@ gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__
         acc += win[1][e] * wt[1][e];
         acc += win[2][e] * wt[2][e];
         acc += v * wt[3][e];
-        out.set(e, acc / (1.f + __expf(-acc)));
+        o[e] = __fdividef(acc, 1.f + __expf(-acc));
         win[0][e] = win[1][e];
         win[1][e] = win[2][e];
         win[2][e] = v;
       }
+      Row<VEC> out;
+      out.set(o);
       out.store(y + (size_t)(t + i) * C);
     }
   }
@@ -529,7 +534,7 @@ __global__ void __launch_bounds__(256, 2) delta_step_kernel(const StepParams p) 
       const float v = from >= 0 ? __bfloat162float(x[(size_t)from * p.ldx]) : (fresh ? 0.f : __bfloat162float(st[from + 3]));
       acc += v * __bfloat162float(w[j]);
     }
-    return __bfloat162float(__float2bfloat16(acc / (1.f + __expf(-acc))));
+    return __bfloat162float(__float2bfloat16(__fdividef(acc, 1.f + __expf(-acc))));
   };
   for (int g = 0; g < G; ++g) {
     const int hv = hk * G + g;

@@ -236,16 +236,21 @@ sample_kernel(const T* __restrict__ logits, int ld, int V, const float* __restri
   if (threadIdx.x == 0) out[r] = a.i < V ? a.i : 0;
 }
 
-// ---- the same sampler with the row held in registers by a cluster of four CTAs ------------------------
-// The single-CTA kernel above re-reads its row from L2 in every bisection pass (about 70 passes over 128 K
-// logits: 1.2 ms for 64 rows).  Here a cluster of SAMPLE_CL CTAs owns a row: CTA c keeps elements
-// [c * seg, (c + 1) * seg) as packed bf16 logits in registers (64 per thread), so a pass is 64 compares per
-// thread, a block reduction and one exchange of a few words over distributed shared memory.  The threshold
-// searches are 4-ary (three thresholds per pass), which halves the number of cluster barriers.  Same
-// thresholds, same Philox noise and same Gumbel-max draw as the single-CTA kernel.
-constexpr int SAMPLE_CL = 4;
+// ---- the same sampler with the row held in registers by a cluster of eight CTAs ------------------------
+// The single-CTA kernel above re-reads its row from L2 in every bisection pass (about 70 passes: 1.2 to 1.9 ms for rows
+// of 151936).  Here a cluster of SAMPLE_CL CTAs owns a row: CTA c keeps elements [c * seg, (c + 1) * seg) as 32-bit keys
+// in registers (NPT per thread), so a pass is NPT compares per thread, a block reduction and one exchange of a few
+// words over distributed shared memory.  The threshold searches are 4-ary (three thresholds per pass), which halves the
+// number of cluster barriers.  Same thresholds, same Philox noise and same Gumbel-max draw as the single-CTA kernel.
+// Eight CTAs, so that a thread has 32 keys of 128 K logits and two CTAs fit an SM.
+constexpr int SAMPLE_CL = 8;
 constexpr int SAMPLE_CT = 512;                    // threads per CTA of the cluster kernel
-constexpr int SAMPLE_NPT = 64;                    // elements per thread: V <= 4 * 512 * 64 = 131072
+constexpr int SAMPLE_LIST = 2048;                 // candidates of a row that the first CTA takes over
+
+__device__ __forceinline__ float2 load_pair(const __nv_bfloat16* p) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+}
+__device__ __forceinline__ float2 load_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
 struct ClusterXchg {
   float f[2][4];                                  // [parity][word]
@@ -291,21 +296,27 @@ __device__ __forceinline__ void block_sum3_i(int& a, int& b, int& c, int* red) {
   }
 }
 
+// Four words of every CTA's slot, one per lane (CTA = lane / 4), summed over the CTAs: lane w gets word w.
+template <typename V>
+__device__ __forceinline__ V lane_of_cluster(uint32_t slot) {
+  static_assert(SAMPLE_CL == 8, "a warp reads the slots of eight CTAs");
+  const int lane = threadIdx.x & 31;
+  const uint32_t addr = mapa_shared(slot, lane >> 2) + 4 * (lane & 3);
+  V v;
+  if constexpr (sizeof(V) == 4 && V(0.5f) != V(0)) v = ld_dsmem_f32(addr); else v = ld_dsmem_s32(addr);
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 8);
+  v += __shfl_xor_sync(0xffffffffu, v, 16);
+  return v;
+}
+
 __device__ __forceinline__ void cluster_sum3_f(float& a, float& b, float& c, ClusterXchg* x, float* red, int& par) {
   block_sum3_f(a, b, c, red);
   if (threadIdx.x == 0) { x->f[par][0] = a; x->f[par][1] = b; x->f[par][2] = c; }
   cluster_arrive_release();
   cluster_wait_acquire();
-  const uint32_t base = smem_u32(&x->f[par][0]);
-  float sa = 0.f, sb = 0.f, sc = 0.f;
-#pragma unroll
-  for (int r = 0; r < SAMPLE_CL; ++r) {
-    const uint32_t ra = mapa_shared(base, r);
-    sa += ld_dsmem_f32(ra);
-    sb += ld_dsmem_f32(ra + 4);
-    sc += ld_dsmem_f32(ra + 8);
-  }
-  a = sa; b = sb; c = sc;
+  float v = lane_of_cluster<float>(smem_u32(&x->f[par][0]));
+  a = __shfl_sync(0xffffffffu, v, 0); b = __shfl_sync(0xffffffffu, v, 1); c = __shfl_sync(0xffffffffu, v, 2);
   par ^= 1;
 }
 __device__ __forceinline__ void cluster_sum3_i(int& a, int& b, int& c, ClusterXchg* x, int* red, int& par) {
@@ -313,16 +324,8 @@ __device__ __forceinline__ void cluster_sum3_i(int& a, int& b, int& c, ClusterXc
   if (threadIdx.x == 0) { x->i[par][0] = a; x->i[par][1] = b; x->i[par][2] = c; }
   cluster_arrive_release();
   cluster_wait_acquire();
-  const uint32_t base = smem_u32(&x->i[par][0]);
-  int sa = 0, sb = 0, sc = 0;
-#pragma unroll
-  for (int r = 0; r < SAMPLE_CL; ++r) {
-    const uint32_t ra = mapa_shared(base, r);
-    sa += ld_dsmem_s32(ra);
-    sb += ld_dsmem_s32(ra + 4);
-    sc += ld_dsmem_s32(ra + 8);
-  }
-  a = sa; b = sb; c = sc;
+  int v = lane_of_cluster<int>(smem_u32(&x->i[par][0]));
+  a = __shfl_sync(0xffffffffu, v, 0); b = __shfl_sync(0xffffffffu, v, 1); c = __shfl_sync(0xffffffffu, v, 2);
   par ^= 1;
 }
 // cluster-wide arg-max of (value, index): smaller index wins ties
@@ -342,10 +345,86 @@ __device__ __forceinline__ ArgMax cluster_argmax(ArgMax a, ClusterXchg* x, ArgMa
   return best;
 }
 
-// bf16 logits only (fp32 rows would not fit the register budget): a thread keeps 32 packed pairs, element j of
-// thread t is row index cr * seg + ((j >> 1) * 512 + t) * 2 + (j & 1).
-__global__ void __launch_bounds__(SAMPLE_CT, 1)
-sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
+__device__ __forceinline__ uint32_t atomic_add_dsmem(uint32_t addr, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+  return old;
+}
+
+// The rest of a draw once the candidates are few: one CTA, a candidate or a few per thread, one barrier per pass.  Masses
+// are summed as integers of 2^-40, so the order of the list (which no one controls) does not matter.
+__device__ __forceinline__ void sample_list(const uint2* list, int n, int k, float pp, uint32_t lowest, const float* uniform,
+                                            int V, unsigned long long seed, unsigned long long step, int r, ArgMax* red,
+                                            unsigned long long (*red64)[16], int* out) {
+  constexpr int M = SAMPLE_LIST / SAMPLE_CT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint2 c[M];                                        // key, index; key 0 is below every threshold
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const int at = threadIdx.x + i * SAMPLE_CT;
+    c[i] = at < n ? list[at] : make_uint2(0u, 0u);
+  }
+  int buf = 0;
+  auto total = [&](unsigned long long v) -> unsigned long long {
+    v = warp_sum(v);
+    if (lane == 0) red64[buf][warp] = v;
+    __syncthreads();
+    v = warp_sum(lane < SAMPLE_CT / 32 ? red64[buf][lane] : 0ull);
+    buf ^= 1;
+    return v;
+  };
+  uint32_t top = 0;
+#pragma unroll
+  for (int i = 0; i < M; ++i) top = max(top, c[i].x);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) red64[0][warp] = top;
+  __syncthreads();
+  top = __reduce_max_sync(0xffffffffu, lane < SAMPLE_CT / 32 ? (uint32_t)red64[0][lane] : 0u);
+  buf = 1;
+  const float mx = key2f(top);
+  uint32_t lo = lowest, hi = top;                    // top-k: the largest key with count(>= key) >= k
+  while (lo < hi) {
+    const uint32_t mid = lo + ((hi - lo) >> 1) + 1;
+    int cnt = 0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) cnt += c[i].x >= mid;
+    if (total((unsigned long long)cnt) >= (unsigned long long)k) lo = mid; else hi = mid - 1;
+  }
+  if (pp < 1.f) {                                    // top-p: the largest key with mass(>= key) >= top_p * mass(>= kth)
+    unsigned long long e[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) e[i] = c[i].x >= lo ? (unsigned long long)(__expf(key2f(c[i].x) - mx) * 1099511627776.f) : 0ull;
+    unsigned long long z = 0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) z += e[i];
+    const double want = (double)pp * (double)total(z);
+    hi = top;
+    while (lo < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1) + 1;
+      unsigned long long m = 0;
+#pragma unroll
+      for (int i = 0; i < M; ++i) m += c[i].x >= mid ? e[i] : 0ull;
+      if ((double)total(m) >= want) lo = mid; else hi = mid - 1;
+    }
+  }
+  ArgMax a{-INFINITY, 0x7fffffff};
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    if (c[i].x >= lo) {
+      const int col = (int)c[i].y;
+      float u = uniform != nullptr ? uniform[(size_t)r * V + col] : uniform_at(seed, step, r, col);
+      u = fminf(fmaxf(u, 1e-20f), 1.f - 1e-7f);
+      a = better(a, ArgMax{key2f(c[i].x) - __logf(-__logf(u)), col});
+    }
+  }
+  a = block_argmax(a, red);
+  if (threadIdx.x == 0) *out = a.i < V ? a.i : 0;
+}
+
+// Element j of thread t is row index cr * seg + ((j >> 1) * 512 + t) * 2 + (j & 1).
+template <typename T, int SAMPLE_NPT>
+__global__ void __launch_bounds__(SAMPLE_CT, SAMPLE_NPT <= 32 ? 2 : 1)
+sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
                       const int* __restrict__ top_k, const float* __restrict__ top_p,
                       const float* __restrict__ uniform, unsigned long long seed, unsigned long long step,
                       const long long* __restrict__ step_ptr, int* __restrict__ out) {
@@ -354,9 +433,13 @@ sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int V, c
   __shared__ float redf[96];
   __shared__ int redi[96];
   __shared__ ClusterXchg xchg;
+  __shared__ uint2 list[SAMPLE_LIST];
+  __shared__ unsigned long long red64[2][16];
+  __shared__ uint32_t list_n, thread_max[SAMPLE_CT];
+  if (threadIdx.x == 0) list_n = 0;
   const int r = blockIdx.x / SAMPLE_CL;
   const int cr = (int)cluster_ctarank();
-  const __nv_bfloat16* row = logits + (size_t)r * ld;
+  const T* row = logits + (size_t)r * ld;
   const float temp = temperature[r];
   const bool greedy = temp <= 1e-5f;
   const float inv_t = greedy ? 1.f : 1.f / temp;
@@ -367,18 +450,18 @@ sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int V, c
   // order-preserving 32-bit keys of the scaled logits; padding holds the key of -inf (KEY_NEG)
   uint32_t key[SAMPLE_NPT];
   const uint32_t KEY_NEG = f2key(-INFINITY);
-  const bool pair_ok = ((reinterpret_cast<uintptr_t>(row) & 3) == 0);
+  const bool pair_ok = reinterpret_cast<uintptr_t>(row) % (2 * sizeof(T)) == 0;
 #pragma unroll
   for (int jj = 0; jj < SAMPLE_NPT / 2; ++jj) {
     const int i = base + jj * 2 * SAMPLE_CT;
     float x0 = -INFINITY, x1 = -INFINITY;
     if (jj * 2 * SAMPLE_CT < seg && i < V) {
       if (pair_ok && i + 1 < V) {
-        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + i));
+        const float2 f = load_pair(row + i);
         x0 = f.x; x1 = f.y;
       } else {
-        x0 = __bfloat162float(row[i]);
-        if (i + 1 < V) x1 = __bfloat162float(row[i + 1]);
+        x0 = load_logit(row, i);
+        if (i + 1 < V) x1 = load_logit(row, i + 1);
       }
     }
     key[2 * jj] = f2key(x0 * inv_t);
@@ -406,6 +489,56 @@ sample_cluster_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int V, c
   const float pp = top_p[r];
   auto sat = [](unsigned long long t) -> uint32_t { return t > 0xffffffffull ? 0xffffffffu : (uint32_t)t; };
 
+  // ---- small k: few elements can be among the k largest.  The k-th largest of a CTA's 512 thread maxima has at least k
+  // elements above or at it, so the largest of these eight keys bounds the k-th value from below.  What lies above goes to
+  // the first CTA as a list, which finishes alone: no pass over the row, no cluster barrier per step.  64 rows of 128256, k =
+  // 50, p = 0.9: 211 us with every step over the row, LIST_US with the list.  Should the list overflow (equal logits), the
+  // steps below do it.
+  if (k < V && k <= SAMPLE_CT) {
+    uint32_t tm = 0;
+#pragma unroll
+    for (int j = 0; j < SAMPLE_NPT; ++j) tm = max(tm, key[j]);
+    thread_max[threadIdx.x] = tm;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      uint32_t v[SAMPLE_CT / 32], lo = 0, hi = 0xffffffffu;
+#pragma unroll
+      for (int i = 0; i < SAMPLE_CT / 32; ++i) v[i] = thread_max[threadIdx.x + 32 * i];
+      while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1) + 1;
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < SAMPLE_CT / 32; ++i) c += v[i] >= mid;
+        if (__reduce_add_sync(0xffffffffu, c) >= k) lo = mid; else hi = mid - 1;
+      }
+      if (threadIdx.x == 0) xchg.i[par][0] = (int)lo;
+    }
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    uint32_t lowest = KEY_NEG + 1;                // (padding is never a candidate)
+#pragma unroll
+    for (int c = 0; c < SAMPLE_CL; ++c) lowest = max(lowest, (uint32_t)ld_dsmem_s32(mapa_shared(smem_u32(&xchg.i[par][0]), c)));
+    par ^= 1;
+    const uint32_t n_addr = mapa_shared(smem_u32(&list_n), 0), list_addr = mapa_shared(smem_u32(list), 0);
+#pragma unroll
+    for (int j = 0; j < SAMPLE_NPT; ++j) {
+      if (key[j] >= lowest) {
+        const uint32_t at = atomic_add_dsmem(n_addr, 1u);
+        if (at < SAMPLE_LIST)
+          asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(list_addr + at * 8), "r"(key[j]), "r"((uint32_t)idx(j))
+                       : "memory");
+      }
+    }
+    cluster_arrive_release();
+    cluster_wait_acquire();
+    const int n = ld_dsmem_s32(n_addr);
+    cluster_arrive_release();                     // the first CTA's memory has been read: the others may leave
+    cluster_wait_acquire();
+    if (n <= SAMPLE_LIST) {
+      if (cr == 0) sample_list(list, n, k, pp, lowest, uniform, V, seed, step, r, red, red64, out + r);
+      return;
+    }
+  }
   // ---- top-k threshold: largest key with count(x >= key) >= k.  Padding (-inf) is never counted: every
   // threshold tried is above KEY_NEG once lo has passed it, and below that the real elements decide.
   uint32_t kth = 0;
@@ -753,8 +886,8 @@ extern "C" int b200_sample(const void* logits, int dtype, int R, int V, int ld, 
                            unsigned long long seed, unsigned long long step, const long long* step_ptr,
                            int* out, cudaStream_t stream) {
   if (R == 0) return 0;
-  if (dtype == 0 && V <= SAMPLE_CL * SAMPLE_CT * SAMPLE_NPT && V >= SAMPLE_CL * SAMPLE_CT * 2 &&
-      sample_cluster_enabled()) {
+  // below 4096 a row is one CTA's business; above 262144 the keys do not fit the registers of a cluster
+  if (V >= 4096 && V <= SAMPLE_CL * SAMPLE_CT * 64 && sample_cluster_enabled()) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(R * SAMPLE_CL);
     cfg.blockDim = dim3(SAMPLE_CT);
@@ -766,8 +899,21 @@ extern "C" int b200_sample(const void* logits, int dtype, int R, int V, int ld, 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, sample_cluster_kernel, (const __nv_bfloat16*)logits, ld, V, temperature,
-                                       top_k, top_p, uniform, seed, step, step_ptr, out));
+    // the fewest keys per thread that hold the row: passes run over all of them
+#define SAMPLE_LAUNCH(T, NPT)                                                                                          \
+  B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, sample_cluster_kernel<T, NPT>, (const T*)logits, ld, V, temperature, top_k, \
+                                     top_p, uniform, seed, step, step_ptr, out))
+#define SAMPLE_SIZES(T)                                                   \
+  do {                                                                    \
+    if (V <= SAMPLE_CL * SAMPLE_CT * 8) SAMPLE_LAUNCH(T, 8);              \
+    else if (V <= SAMPLE_CL * SAMPLE_CT * 32) SAMPLE_LAUNCH(T, 32);       \
+    else if (V <= SAMPLE_CL * SAMPLE_CT * 40) SAMPLE_LAUNCH(T, 40);       \
+    else SAMPLE_LAUNCH(T, 64);                                            \
+  } while (0)
+    if (dtype == 0) SAMPLE_SIZES(__nv_bfloat16);
+    else SAMPLE_SIZES(float);
+#undef SAMPLE_SIZES
+#undef SAMPLE_LAUNCH
     return 0;
   }
   if (dtype == 0)
