@@ -143,3 +143,27 @@ def test_experts_with_biases_oai_swiglu_and_padded_hidden(packed):
     want = ref.moe_experts(x, w13, w2, ids, wt, 0, act=act, b13=b13, b2=b2)
     err = (got.float() - want.float()).abs().max().item()
     assert err <= 3e-2 * want.float().abs().max().item() + 2e-2, err
+
+
+# slices of the eight CTAs of the plan: fewer entries than CTAs, ragged slices, one expert, more experts than threads, experts
+# of other ranks on both sides
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,k,E,lo,local", [(1, 1, 4, 0, 4), (1, 3, 5, 1, 2), (7, 8, 33, 0, 33), (501, 5, 130, 17, 100),
+                                            (300, 2, 1, 0, 1), (2000, 4, 8191, 0, 8191), (4096, 8, 128, 64, 64)])
+def test_permutation_plan_over_the_cluster(T, k, E, lo, local):
+    from vllm_torchtpu_b200.ops import cuda
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.randint(0, E, (T, k), generator=g, device="cuda", dtype=torch.int32)
+    x = torch.randn(T, 24, generator=g, device="cuda").bfloat16()
+    x_perm, off, src, inv = cuda.moe_permute(x, ids, lo, local)
+    here = (ids >= lo) & (ids < lo + local)
+    counts = torch.bincount((ids[here] - lo).long(), minlength=local)
+    assert torch.equal(off.long(), torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
+    n = int(off[-1])
+    inv = inv.view(T, k).long()
+    assert inv[~here].eq(-1).all() and torch.equal(inv[here].sort().values, torch.arange(n, device="cuda"))
+    # every entry lies in its expert's rows and comes from its token
+    group = torch.bucketize(inv[here], off[1:].long(), right=True)
+    assert torch.equal(group, (ids[here] - lo).long())
+    token = torch.arange(T, device="cuda")[:, None].expand(T, k)[here]
+    assert torch.equal(src[inv[here]].long(), token) and torch.equal(x_perm[inv[here]], x[token])

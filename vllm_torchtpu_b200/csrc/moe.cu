@@ -117,30 +117,72 @@ __global__ void moe_route_kernel(const T* __restrict__ logits, int ld, int Tn, i
   }
 }
 
-// One CTA.  entries = T * k.  Experts outside [e_lo, e_lo + E_local) are not local (inv_pos = -1).
-__global__ void __launch_bounds__(1024)
+// One cluster of eight CTAs, each with an eighth of the entries (T * k): counts per expert, their sums over the cluster through
+// distributed shared memory, positions behind those of the lower CTAs.  Experts outside [e_lo, e_lo + E_local) are not
+// local (inv_pos = -1).  Bound by the latency of the passes over the entries and their shared-memory atomics, which one
+// CTA with a serial sum over the experts took 37 us for at 32768 entries and 128 experts.
+constexpr int PLAN_CTAS = 8, PLAN_THREADS = 1024, PLAN_EXPERTS = 8192;
+__global__ void __cluster_dims__(PLAN_CTAS, 1, 1) __launch_bounds__(PLAN_THREADS)
 moe_permute_plan_kernel(const int* __restrict__ ids, int entries, int top_k, int e_lo, int E_local,
                         int* __restrict__ group_off, int* __restrict__ row_src, int* __restrict__ inv_pos) {
   extern __shared__ int s_cnt[];                 // [E_local + 1] counts, then cursors
-  for (int e = threadIdx.x; e <= E_local; e += blockDim.x) s_cnt[e] = 0;
+  const int rank = (int)cluster_ctarank(), tid = threadIdx.x;
+  const int per = (entries + PLAN_CTAS - 1) / PLAN_CTAS, begin = min(entries, rank * per), end = min(entries, begin + per);
+  for (int e = tid; e <= E_local; e += PLAN_THREADS) s_cnt[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
+#pragma unroll 4
+  for (int i = begin + tid; i < end; i += PLAN_THREADS) {
     const int e = ids[i] - e_lo;
     if (e >= 0 && e < E_local) atomicAdd(&s_cnt[e], 1);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int e = 0; e < E_local; ++e) {
-      const int c = s_cnt[e];
-      group_off[e] = run;
-      s_cnt[e] = run;                            // becomes the cursor
-      run += c;
+  cluster_arrive_release();
+  cluster_wait_acquire();
+  int below[PLAN_EXPERTS / PLAN_THREADS], all[PLAN_EXPERTS / PLAN_THREADS];
+#pragma unroll
+  for (int x = 0; x < PLAN_EXPERTS / PLAN_THREADS; ++x) {
+    const int e = tid + x * PLAN_THREADS;
+    below[x] = all[x] = 0;
+    if (e < E_local) {
+#pragma unroll
+      for (int r = 0; r < PLAN_CTAS; ++r) {
+        int c;
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(c) : "r"(mapa_shared(smem_u32(&s_cnt[e]), r)) : "memory");
+        all[x] += c;
+        if (r < rank) below[x] += c;
+      }
     }
-    group_off[E_local] = run;
+  }
+  cluster_arrive_release();                      // every count has been read
+  cluster_wait_acquire();
+#pragma unroll
+  for (int x = 0; x < PLAN_EXPERTS / PLAN_THREADS; ++x)
+    if (tid + x * PLAN_THREADS < E_local) s_cnt[tid + x * PLAN_THREADS] = all[x];
+  __syncthreads();
+  if (tid < 32) {                                // sums in front of every expert
+    int run = 0;
+    for (int b = 0; b < E_local; b += 32) {
+      const int n = b + tid < E_local ? s_cnt[b + tid] : 0;
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (tid >= o) incl += v;
+      }
+      if (b + tid < E_local) {
+        s_cnt[b + tid] = run + incl - n;
+        if (rank == 0) group_off[b + tid] = run + incl - n;
+      }
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (rank == 0 && tid == 0) group_off[E_local] = run;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < entries; i += blockDim.x) {
+#pragma unroll
+  for (int x = 0; x < PLAN_EXPERTS / PLAN_THREADS; ++x)
+    if (tid + x * PLAN_THREADS < E_local) s_cnt[tid + x * PLAN_THREADS] += below[x];
+  __syncthreads();
+#pragma unroll 4
+  for (int i = begin + tid; i < end; i += PLAN_THREADS) {
     const int e = ids[i] - e_lo;
     int pos = -1;
     if (e >= 0 && e < E_local) {
@@ -388,8 +430,8 @@ extern "C" int b200_moe_permute(const void* x, const int* ids, int T, int top_k,
     b200_set_last_error("moe_permute: at most 8191 experts, rows of an even number of bytes", __FILE__, __LINE__);
     return -1;
   }
-  moe_permute_plan_kernel<<<1, 1024, (E_local + 1) * sizeof(int), stream>>>(ids, T * top_k, top_k, e_lo,
-                                                                           E_local, group_off, row_src, inv_pos);
+  moe_permute_plan_kernel<<<PLAN_CTAS, PLAN_THREADS, (E_local + 1) * sizeof(int), stream>>>(
+      ids, T * top_k, top_k, e_lo, E_local, group_off, row_src, inv_pos);
   int blocks = T * top_k;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (row_bytes % 16 == 0 && ((uintptr_t)x | (uintptr_t)x_perm) % 16 == 0)
