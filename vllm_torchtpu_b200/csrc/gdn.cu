@@ -41,7 +41,8 @@ struct Row<8> {
 // to 32 tokens of one request and 128 * VEC channels, with the three tokens in front of them.  Bound by memory: one read
 // and one write of the rows; eight rows of a thread are in flight.  Only the CTA of a request's first tokens touches
 // the carried window: it reads the old one and writes the new one.  Rows of no request become zeros.
-// (One thread per channel walking all tokens of the request took about 2.2 ms for 4 x 2048 tokens and 8192 channels.)
+// 4 x 2048 tokens and 8192 channels take 100 us (2.7 TB/s): the exponential
+// and the reciprocal of every value.  One thread per channel through all tokens of a request had one load in flight.
 template <int VEC>
 __global__ void __launch_bounds__(128)
 gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, __nv_bfloat16* conv_pool,

@@ -12,6 +12,10 @@
 //     K^T U
 // Everything that is fp32 (S, T, M, R, U) enters as three bf16 parts, which hold its 24 bits; an exact bf16 factor makes three
 // products, two split ones six (what is left out is below 2^-24).  Sums are fp32.
+//
+// What bounds it: the chain of a request, 64 tokens at a time (6.4 us a chunk: 3840 cycles of products, the rest splits and
+// barriers between them); token by token (gdn_recurrent_kernel) a token takes 0.67 us.  4 x 2048 tokens, 32 value heads:
+// 1369 us there, 180 + 205 us here.
 #include <cstring>
 #include <type_traits>
 

@@ -492,7 +492,7 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
   // ---- small k: few elements can be among the k largest.  The k-th largest of a CTA's 512 thread maxima has at least k
   // elements above or at it, so the largest of these eight keys bounds the k-th value from below.  What lies above goes to
   // the first CTA as a list, which finishes alone: no pass over the row, no cluster barrier per step.  64 rows of 128256, k =
-  // 50, p = 0.9: 211 us with every step over the row, LIST_US with the list.  Should the list overflow (equal logits), the
+  // 50, p = 0.9: 211 us with every step over the row, 70 with the list.  Should the list overflow (equal logits), the
   // steps below do it.
   if (k < V && k <= SAMPLE_CT) {
     uint32_t tm = 0;
