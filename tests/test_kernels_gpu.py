@@ -76,7 +76,7 @@ def test_rope_and_cache(D, interleaved, qk_norm):
 
 
 def _attn_case(q_lens, ctx_lens, Hq, Hkv, D, bs=16, window=None, softcap=None, sinks=False, num_decode=0,
-               kv_fp8=False):
+               kv_fp8=False, scales=(0.02, 0.03)):
     g = torch.Generator(device=DEV).manual_seed(2)
     R = len(q_lens)
     seq = [q + c for q, c in zip(q_lens, ctx_lens)]
@@ -86,7 +86,7 @@ def _attn_case(q_lens, ctx_lens, Hq, Hkv, D, bs=16, window=None, softcap=None, s
     k_scale, v_scale = 1.0, 1.0
     if kv_fp8:
         # e4m3 cache with per-tensor scales: the oracle dequantises the same bytes in fp32
-        k_scale, v_scale = 0.02, 0.03
+        k_scale, v_scale = scales
         cache = torch.stack([cache[:, 0].float() / k_scale, cache[:, 1].float() / v_scale],
                             1).to(torch.float8_e4m3fn)
     perm = (torch.randperm(nb - 1, device=DEV) + 1).to(torch.int32)
@@ -147,6 +147,15 @@ def test_attention_fp8_kv_cache(Hq, Hkv, D):
     _attn_case([1, 1, 200, 64, 65, 1, 333], [40, 900, 0, 128, 37, 0, 1000], Hq, Hkv, D, num_decode=2,
                kv_fp8=True)
     _attn_case([1, 130, 17], [500, 300, 0], Hq, Hkv, D, window=128, sinks=True, num_decode=1, kv_fp8=True)
+
+
+# prompts over an e4m3 cache with values of scale one: pages expanded for the tcgen05 kernel.  Pages of 16 and 32, lengths that
+# end a page, requests of one token behind and between, no decode range
+@pytest.mark.parametrize("Hq,Hkv,bs,kw", [(32, 8, 16, {}), (8, 8, 16, dict(softcap=20.0)), (8, 1, 32, dict(sinks=True))])
+def test_attention_fp8_kv_cache_expanded_for_prompts(Hq, Hkv, bs, kw):
+    _attn_case([1, 200, 1, 16, 333, 400], [33, 0, 70, 16, 1000, 1500], Hq, Hkv, 128, num_decode=1, kv_fp8=True, scales=(0.7, 1.0),
+               bs=bs, **kw)
+    _attn_case([3, 700], [1532, 0], Hq, Hkv, 128, num_decode=0, kv_fp8=True, scales=(1.0, 1.0), bs=bs, **kw)
 
 
 def test_attention_window_softcap_sinks():

@@ -681,13 +681,15 @@ def paged_attention(q, kv_cache, meta, scale, *, sliding_window=None, softcap=No
                 c_int(max_blocks), c_int(bs), c_longlong(nb), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale),
                 c_float(cap), c_int(meta.dcp_size), c_int(meta.dcp_rank), c_int(meta.dcp_interleave), _stream()),
                 "attn_prefill_dcp")
-        elif D == 128 and G in (1, 2, 4, 8) and envs.B200_ATTN_PREFILL_IMPL == "tc" and not kv_fp8:
-            # tcgen05 kernel: one CTA per (kv head, 128 / G positions), K/V shared by the GQA group
+        elif (D == 128 and G in (1, 2, 4, 8) and envs.B200_ATTN_PREFILL_IMPL == "tc"
+              and (not kv_fp8 or (wide := _expanded_pages(kv_cache, meta, nd, R, (T - nd) * Hq, window, v_scale)) is not None)):
+            # tcgen05 kernel: 128 / G positions of a kv head per tile, K/V shared by the GQA group
+            pool, table = wide if kv_fp8 else (kv_cache, meta.block_tables)
             _check(L.b200_attn_prefill_tc(
-                _p(q), _p(kv_cache), _p(out), _p(lse), _p(meta.block_tables), _p(meta.seq_lens),
-                _p(meta.query_start_loc), c_int(nd), c_int(R), c_int(tiles), c_int(T), c_int(max_blocks),
-                c_int(bs), c_longlong(nb), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale), c_int(window),
-                c_float(cap), _p(sinks), c_int(ldo), _p(ws.status), _stream()), "attn_prefill_tc")
+                _p(q), _p(pool), _p(out), _p(lse), _p(table), _p(meta.seq_lens),
+                _p(meta.query_start_loc), c_int(nd), c_int(R), c_int(tiles), c_int(T), c_int(table.shape[1]),
+                c_int(bs), c_longlong(pool.shape[0]), c_int(Hq), c_int(Hkv), c_int(D), c_float(scale * k_scale if kv_fp8 else scale),
+                c_int(window), c_float(cap), _p(sinks), c_int(ldo), c_int(kv_fp8), _p(ws.status), _stream()), "attn_prefill_tc")
         else:
             args = (_p(q), _p(kv_cache), _p(out), _p(lse), _p(meta.block_tables), _p(meta.seq_lens),
                     _p(meta.query_start_loc), c_int(nd), c_int(R), c_int(tiles), c_int(max_blocks), c_int(bs),
@@ -702,6 +704,29 @@ def paged_attention(q, kv_cache, meta, scale, *, sliding_window=None, softcap=No
     if return_lse:
         return out, lse
     return out
+
+
+def _expanded_pages(kv_cache, meta, nd: int, R: int, heads_rows: int, window: int, v_scale: float):
+    """Prompts over an e4m3 cache on the tcgen05 kernel, which reads 16-bit pages: the pages of requests nd .. R - 1
+    expanded (exactly) into a pool of this call, with its block table.  None where the mma.sync kernel, which expands in
+    registers, has to do it: lengths unknown to the host, a window (few of the pages would be read), a scale of the values
+    (it goes to the output there), pools above 1 GB; and where it is as fast, because the call is short and the second
+    launch and its tensors cost 15 us: 4.4 M (query head, key) pairs took 43 us there and 58 this way, 9.8 M 76 and 57."""
+    if (meta.seq_lens_cpu is None or window or v_scale != 1.0 or heads_rows * (meta.max_seq_len or 0) < 8_000_000
+            or kv_cache.data_ptr() % 16 or torch.cuda.is_current_stream_capturing()):
+        return None
+    nb, _, Hkv, bs, D = kv_cache.shape
+    longest = int(meta.seq_lens_cpu[nd:R].max())
+    pages = -(-longest // bs)
+    if pages <= 0 or heads_rows * longest < 8_000_000 or bs % 16 or (R - nd) * pages * 2 * Hkv * bs * D > 1 << 29:
+        return None
+    pool = torch.empty(((R - nd) * pages, 2, Hkv, bs, D), dtype=torch.bfloat16, device=kv_cache.device)
+    table = torch.empty((R, pages), dtype=torch.int32, device=kv_cache.device)
+    _check(lib().b200_expand_e4m3_pages(
+        _p(kv_cache), _p(pool), _p(table), _p(meta.block_tables), _p(meta.seq_lens), c_int(nd), c_int(R - nd), c_int(pages),
+        c_int(meta.block_tables.shape[1]), c_int(bs), c_longlong(nb), c_int(Hkv), _stream()), "expand_e4m3_pages")
+    count_launch()
+    return pool, table
 
 
 def _out_rows(q, out, tensor_cores: bool = False) -> int:
