@@ -130,3 +130,25 @@ def test_decays_that_underflow():
     want = g.gdn_forward(mixed, a, b, None, meta, *pools[1], conv_w, A_log, dt, Hk, Hv, dk, dv)
     assert (got.float() - want.float()).abs().max() <= 2e-2 * want.float().abs().max()
     assert (pools[0][1] - pools[1][1]).abs().max() <= 2e-2 * pools[1][1].abs().max()
+
+
+def test_silu_of_large_negative_values():
+    """silu(-88) is -5.3e-37, a normal bf16 number: 1 + exp(88) is below the largest fp32 number but above 2^126, where the
+    approximate division returns zero."""
+    from vllm_torchtpu_b200.ops import cuda
+    Hk, Hv, D = 1, 2, 128
+    C = (2 * Hk + Hv) * D
+    conv_w = torch.zeros(C, 4, device=DEV).bfloat16()
+    conv_w[:, 3] = 1
+    x = torch.full((40, C), -88.0, device=DEV).bfloat16()
+    want = -88.0 / (1.0 + torch.exp(torch.tensor(88.0, dtype=torch.float64))).item()
+    y = cuda.short_conv(x, _meta([33, 1, 6], [0, 0, 0], [0, 1, 2]), torch.zeros(3, C, 3, device=DEV, dtype=torch.bfloat16), conv_w)
+    # (2^-9 for bf16, 2^-16 for the exponential's argument: 88 * log2(e) in fp32)
+    torch.testing.assert_close(y.double() / want, torch.ones_like(y, dtype=torch.float64), rtol=0, atol=2 ** -8)
+    # single tokens: o = (q k) v, q = k of unit length but for dk^-1/2, beta = 1, state from zero
+    x[:, :2 * Hk * D] = 5.0
+    big = torch.full((1, Hv), 30.0, device=DEV).bfloat16()
+    rec = torch.zeros(1, Hv, D, D, device=DEV)
+    o = cuda.gdn_forward(x[:1], big, big, _meta([1], [0], [0]), torch.zeros(1, C, 3, device=DEV, dtype=torch.bfloat16), rec, conv_w,
+                         torch.zeros(Hv, device=DEV), torch.zeros(Hv, device=DEV), Hk, Hv, D, D)
+    torch.testing.assert_close(o.double() / (want * D ** -0.5), torch.ones_like(o, dtype=torch.float64), rtol=0, atol=2 ** -7)

@@ -160,7 +160,7 @@ gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__
         acc += win[1][e] * wt[1][e];
         acc += win[2][e] * wt[2][e];
         acc += v * wt[3][e];
-        o[e] = __fdividef(acc, 1.f + __expf(-acc));
+        o[e] = acc / (1.f + __expf(-acc));
         win[0][e] = win[1][e];
         win[1][e] = win[2][e];
         win[2][e] = v;
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(256, 2) delta_step_kernel(const StepParams p) 
       const float v = from >= 0 ? __bfloat162float(x[(size_t)from * p.ldx]) : (fresh ? 0.f : __bfloat162float(st[from + 3]));
       acc += v * __bfloat162float(w[j]);
     }
-    return __bfloat162float(__float2bfloat16(__fdividef(acc, 1.f + __expf(-acc))));
+    return __bfloat162float(__float2bfloat16(acc / (1.f + __expf(-acc))));
   };
   for (int g = 0; g < G; ++g) {
     const int hv = hk * G + g;
