@@ -152,3 +152,37 @@ def test_silu_of_large_negative_values():
     o = cuda.gdn_forward(x[:1], big, big, _meta([1], [0], [0]), torch.zeros(1, C, 3, device=DEV, dtype=torch.bfloat16), rec, conv_w,
                          torch.zeros(Hv, device=DEV), torch.zeros(Hv, device=DEV), Hk, Hv, D, D)
     torch.testing.assert_close(o.double() / (want * D ** -0.5), torch.ones_like(o, dtype=torch.float64), rtol=0, atol=2 ** -7)
+
+
+@pytest.mark.parametrize("what", ["gate", "beta", "key", "query", "value", "value inf", "huge key"])
+def test_values_that_are_not_finite_reach_no_token_in_front_of_them(what):
+    """Chunks of 64 tokens: what is not finite in token 70 shows in the outputs and states that it reaches token by token, and
+    nowhere else.  A key whose square leaves the range of fp32 counts as a zero vector."""
+    from vllm_torchtpu_b200.ops import cuda
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    Hk, Hv, D = 2, 4, 128
+    q_lens, ctx, slots = [150, 70, 20], [0, 30, 5], [2, 0, 1]
+    T, C, at = sum(q_lens), (2 * Hk + Hv) * D, 70
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)                      # noqa: E731
+    mixed, a, b = rnd(T, C).bfloat16(), rnd(T, Hv).bfloat16(), rnd(T, Hv).bfloat16()
+    conv_w = (rnd(C, 4) * 0.3).bfloat16()
+    conv_w[:, 3] = 0.5
+    A_log, dt = rnd(Hv) * 0.3, rnd(Hv) * 0.3
+    nan, inf = float("nan"), float("inf")
+    if what == "gate":
+        a[at, 1] = nan
+    elif what == "beta":
+        b[at, 1] = nan
+    else:
+        col = {"query": D + 7, "key": (Hk + 1) * D + 7, "huge key": (Hk + 1) * D + 7}.get(what, (2 * Hk + 1) * D + 7)
+        mixed[at, col] = {"value inf": inf, "huge key": 1e20}.get(what, nan)
+    meta = _meta(q_lens, ctx, slots)
+    conv, rec = rnd(3, C, 3).bfloat16(), rnd(3, Hv, D, D) * 0.1
+    got_pools, want_pools = [conv.clone(), rec.clone()], [conv.clone(), rec.clone()]
+    got = cuda.gdn_forward(mixed, a, b, meta, *got_pools, conv_w, A_log, dt, Hk, Hv, D, D)
+    want = g.gdn_forward(mixed, a, b, None, meta, *want_pools, conv_w, A_log, dt, Hk, Hv, D, D)
+    for x, y in ((got, want), (got_pools[1], want_pools[1])):
+        assert torch.equal(torch.isfinite(x), torch.isfinite(y))
+        x, y = (t.float().nan_to_num(0.0, 0.0, 0.0) for t in (x, y))
+        assert (x - y).abs().max() <= 2e-2 * y.abs().max() + 1e-3
+    assert torch.isfinite(want[:at]).all() and cuda.check_status() == 0

@@ -25,7 +25,8 @@ namespace b200 {
 namespace gdnc {
 
 constexpr int C = 64, D = 128;
-constexpr int UNIT = 128 * 64 + 3 * 64 + 64;          // floats per (chunk, head): [T; M], row factors of k S, q S and U, decay
+constexpr int FACTORS = 128 * 64;                     // floats of a (chunk, head): [T; M], row factors of k S, q S and U, decay
+constexpr int UNIT = FACTORS + 4 * 64;                // and a flag
 
 struct Params {
   const __nv_bfloat16 *y, *a, *b;                     // y: convolved rows [T, Cy]
@@ -105,7 +106,8 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const Params p) {
         z = -ea * (av > 20.f ? av : log1pf(__expf(av)));
         be = 1.f / (1.f + __expf(-__bfloat162float(p.b[(size_t)(row0 + t) * p.lda + hv])));
       }
-      g[e] = (double)fmaxf(z, -1000.f);               // (2^-1000 is zero in fp32; differences of sums stay finite)
+      z = z < -1000.f ? -1000.f : z;                  // (2^-1000 is zero in fp32; differences of sums stay finite; a NaN stays)
+      g[e] = (double)z;
       sbeta[t] = be;
     }
     double s = g[0] + g[1];
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const Params p) {
     sG[2 * lane + 1] = s;
   }
   __syncthreads();
+  int odd;                                            // (see token_by_token)
   {
     float s = 0.f;                                    // thread = row of the tile
 #pragma unroll 4
@@ -131,6 +134,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const Params p) {
       }
     }
     sik[tid] = (tid < C ? 1.f : rsqrtf((float)D)) / fmaxf(sqrtf(s), 1e-12f);
+    odd = !isfinite(s) || (tid < C && !isfinite(sbeta[tid] + (float)sG[tid]));
   }
   float kk[8][4], qk[8][4];
 #pragma unroll
@@ -169,7 +173,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const Params p) {
       sP[i * LDA + j] = sik[C + i] * d * qk[nb][e];
     }
   }
-  __syncthreads();
+  odd = __syncthreads_or(odd);
   // ---- (I + A)^-1 in place of A: blocks of 16 by substitution (a thread a column), then two levels of
   // [T1 0; -T2 A21 T1  T2]
   if (tid < C) {
@@ -273,12 +277,15 @@ __global__ void __launch_bounds__(128) gdn_chunk_kernel(const Params p) {
   }
   if (tid < C) {
     const int i = tid;
-    float* f = unit + 2 * C * C;
+    float* f = unit + FACTORS;
     const float e = exp2f((float)sG[i]);
     f[i] = sik[i] * e;
     f[C + i] = sik[C + i] * e;
     f[2 * C + i] = sik[i] * exp2f((float)(sG[C - 1] - sG[i]));
-    if (i == 0) f[3 * C] = exp2f((float)sG[C - 1]);
+    if (i == 0) {
+      f[3 * C] = exp2f((float)sG[C - 1]);
+      f[3 * C + 1] = odd ? 1.f : 0.f;
+    }
   }
 }
 
@@ -338,9 +345,69 @@ __device__ __forceinline__ void put32(uint8_t* row128, int sw, int which, uint32
   }
 }
 
+// The rule token by token, for the rest of a request from a chunk on that holds a value that is not finite: in the products
+// of a chunk that value would reach the tokens in front of it as 0 * NaN.  (Sums of finite squares in fp32 bound the products
+// of q and k; what overflows there counts as not finite.)  Thread = (row ln of the state, 64 of its columns); k S and q S are
+// summed over the lanes of a warp (afterwards lane l has columns 2 l and 2 l + 1), then over the four warps of a half.
+__device__ __noinline__ void token_by_token(const Params& p, float* red, int qs, int n, int hv, int hk, float* st) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ln = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 64;
+  float *rqk = red + 8 * 128, *su = rqk + 4 * 3;      // [8 warps][2][64]; q k, k k, q q of four warps; u
+  const float ea = __expf(p.A_log[hv]), dt = p.dt_bias[hv];
+  float S[64];
+#pragma unroll
+  for (int i = 0; i < 64; ++i) S[i] = st[i];
+  auto lanes_sum = [&](float factor) -> float2 {
+    float a[32];
+    const bool up = lane & 16;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      a[i] = factor * (up ? S[32 + i] : S[i]) + __shfl_xor_sync(0xffffffffu, factor * (up ? S[i] : S[32 + i]), 16);
+#pragma unroll
+    for (int h = 16; h >= 2; h >>= 1) {
+      const bool hi = lane & (h >> 1);
+#pragma unroll
+      for (int i = 0; i < h; ++i) a[i] = (hi ? a[h + i] : a[i]) + __shfl_xor_sync(0xffffffffu, hi ? a[i] : a[h + i], h >> 1);
+    }
+    return make_float2(a[0], a[1]);
+  };
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    const __nv_bfloat16* y = p.y + (size_t)(qs + t) * p.Cy;
+    float kv = __bfloat162float(y[(p.Hk + hk) * D + ln]), qv = __bfloat162float(y[hk * D + ln]);
+    const float kk = warp_sum(kv * kv), qq = warp_sum(qv * qv);
+    if (warp < 4 && lane == 0) { rqk[4 + warp] = kk; rqk[8 + warp] = qq; }
+    __syncthreads();
+    auto over_warps = [&](int i) -> float { return (rqk[4 * i] + rqk[4 * i + 1]) + (rqk[4 * i + 2] + rqk[4 * i + 3]); };
+    kv *= 1.f / fmaxf(sqrtf(over_warps(1)), 1e-12f);
+    qv *= rsqrtf((float)D) / fmaxf(sqrtf(over_warps(2)), 1e-12f);
+    const float z = __bfloat162float(p.a[(size_t)(qs + t) * p.lda + hv]) + dt;
+    const float dec = __expf(-ea * (z > 20.f ? z : log1pf(__expf(z))));
+    const float beta = 1.f / (1.f + __expf(-__bfloat162float(p.b[(size_t)(qs + t) * p.lda + hv])));
+#pragma unroll
+    for (int i = 0; i < 64; ++i) S[i] *= dec;
+    reinterpret_cast<float2*>(red + warp * 128)[lane] = lanes_sum(kv);
+    reinterpret_cast<float2*>(red + warp * 128 + 64)[lane] = lanes_sum(qv);
+    const float d = warp_sum(kv * qv);
+    if (warp < 4 && lane == 0) rqk[warp] = d;
+    __syncthreads();
+    if (tid < D) {                                    // thread = value column
+      const float* x = red + (tid >> 6) * 512 + (tid & 63);
+      const float mem = (x[0] + x[128]) + (x[256] + x[384]), o = (x[64] + x[192]) + (x[320] + x[448]);
+      const float u = (__bfloat162float(y[(2 * p.Hk + hv) * D + tid]) - mem) * beta;
+      su[tid] = u;
+      p.out[((size_t)(qs + t) * p.Hv + hv) * D + tid] = __float2bfloat16(fmaf(over_warps(0), u, o));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 64; ++i) S[i] = fmaf(kv, su[c0 + i], S[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 64; ++i) st[i] = S[i];
+}
+
 // grid (Hv, R), 256 threads: thread = (lane of the tensor memory, half of the 128 value columns).  Lanes 0-63 are the
 // chunk's tokens as keys, lanes 64-127 as queries; for the state they are its 128 rows, held in registers.
-__global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const Params p) {
+__global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   if (smem + SMEM_USED > smem_raw + SMEM_TOTAL) {     // (the base is 1024-byte aligned: nothing is cut off)
@@ -390,9 +457,9 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const Params p) {
       const uint32_t d = dst + (ch >> 3) * (128 * 128) + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(t < n ? 16 : 0) : "memory");
     }
-    // row factors and the decay: 193 floats
+    // row factors, the decay and the flag: 194 floats
     if (tid < 49) {
-      const float* src = unit + (size_t)c * unit_step + 2 * C * C + tid * 4;
+      const float* src = unit + (size_t)c * unit_step + FACTORS + tid * 4;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(fac + (c & 1) * 256 + tid * 4)), "l"(src) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -456,8 +523,9 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const Params p) {
   constexpr uint32_t idesc_ab = umma_idesc_bf16(128, 128) | (1u << 16) | (1u << 15);        // A M-major too
   const uint64_t s_desc = desc_sw128(smem_u32(smem + SMEM_S), PANEL_S), r_desc = desc_sw128(smem_u32(smem + SMEM_R), PANEL_R);
   uint32_t phase = 0;
-  bool ok = true;
-  for (int c = 0; c < chunks; ++c) {
+  bool ok = true, odd = false;
+  int c = 0;
+  for (; c < chunks; ++c) {
     const float* f = fac + (c & 1) * 256;
     const uint32_t kq = smem_u32(smem + SMEM_KQ + (c & 1) * KQ_BYTES);
     fence_proxy_async_smem();
@@ -477,6 +545,20 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const Params p) {
     }
     __syncwarp();
     if (c + 1 < chunks) load_kq(c + 1);
+    odd = f[3 * C + 1] != 0.f;
+    {                                                 // the pieces of V that this thread has copied: 0 * infinity is a NaN
+      const __nv_bfloat162 z = __float2bfloat162_rn(0.f);
+      __nv_bfloat162 s[4] = {z, z, z, z};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint4 q = *reinterpret_cast<const uint4*>(smem + SMEM_V + (tid + i * 256) * 16);
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[e] = __hfma2(h[e], z, s[e]);
+      }
+      const float2 sum = __bfloat1622float2(__hadd2(__hadd2(s[0], s[1]), __hadd2(s[2], s[3])));
+      odd |= !(sum.x + sum.y == 0.f);
+    }
     ok = mbar_wait(bar, phase, abort_flag, p.status, ST_TIMEOUT_TMEM_FULL) && ok;
     phase ^= 1;
     tc_fence_after();
@@ -503,7 +585,7 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const Params p) {
     }
     fence_proxy_async_smem();
     tc_fence_before();
-    if (__syncthreads_or(!ok)) break;
+    if (__syncthreads_or(!ok || odd)) break;          // (the state is still that in front of the chunk)
     if (warp == 0 && elect_one()) {                   // [T; M] R
       tc_fence_after();
       constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};                 // small products first
@@ -606,11 +688,13 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const Params p) {
     for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(st + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
   }
   tc_fence_before();
-  __syncthreads();
+  odd = __syncthreads_or(odd);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  if (odd && !__syncthreads_or(!ok))
+    token_by_token(p, reinterpret_cast<float*>(smem), qs + c * C, n - c * C, hv, hk, st);
 }
 
 }  // namespace gdnc
