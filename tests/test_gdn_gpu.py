@@ -186,3 +186,29 @@ def test_values_that_are_not_finite_reach_no_token_in_front_of_them(what):
         x, y = (t.float().nan_to_num(0.0, 0.0, 0.0) for t in (x, y))
         assert (x - y).abs().max() <= 2e-2 * y.abs().max() + 1e-3
     assert torch.isfinite(want[:at]).all() and cuda.check_status() == 0
+
+
+@pytest.mark.parametrize("off", [1, 2])
+@pytest.mark.parametrize("q_lens,ctx", [([1, 1, 1], [0, 4, 9]), ([5, 1, 40], [3, 7, 0])])
+def test_states_at_any_address(q_lens, ctx, off):
+    """Pools that begin on 4 or 8 bytes are taken by the kernels that read single floats or pairs."""
+    from vllm_torchtpu_b200.ops import cuda
+    gen = torch.Generator(device=DEV).manual_seed(10)
+    Hk, Hv, D, R, T = 2, 4, 128, len(q_lens), sum(q_lens)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)                      # noqa: E731
+    C = (2 * Hk + Hv) * D
+    mixed, a, ac, b = rnd(T, C).bfloat16(), rnd(T, Hv).bfloat16(), rnd(T, Hv, D).bfloat16(), rnd(T, Hv).bfloat16()
+    conv_w, A_log, dt, dtc = (rnd(C, 4) * 0.3).bfloat16(), rnd(Hv) * 0.3, rnd(Hv) * 0.3, rnd(Hv, D) * 0.3
+    conv, rec = rnd(R, C, 3).bfloat16(), rnd(R, Hv, D, D) * 0.1
+    meta = _meta(q_lens, ctx, list(range(R)))
+    apart = torch.empty(rec.numel() + 4, device=DEV)[off:off + rec.numel()].view_as(rec)
+    assert apart.data_ptr() % 16 == 4 * off
+    q, k, v = (t.reshape(T, -1, D) for t in mixed.split([Hk * D, Hk * D, Hv * D], -1))
+    for call in (lambda st: cuda.gdn_forward(mixed, a, b, meta, conv.clone(), st, conv_w, A_log, dt, Hk, Hv, D, D),
+                 lambda st: cuda.kda_forward(q, k, v, ac, b, meta, st, A_log, dtc)):
+        want_rec = rec.clone()
+        apart.copy_(rec)
+        got, want = call(apart), call(want_rec)
+        # fp32 sums of 128 products in another order (2^-24 * sqrt(128) * a few), bf16 outputs
+        torch.testing.assert_close(apart, want_rec, rtol=1e-4, atol=1e-5)
+        torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -7, atol=1e-4)

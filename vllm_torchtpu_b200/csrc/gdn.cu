@@ -333,7 +333,7 @@ gdn_recurrent_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
   // S[c][2 x], S[c][2 x + 1]: rows 4 (PARTS x + part) + 0 .. 3 of column j + c
   uint64_t S[2][16];
   float* sp = rec_pool + (((size_t)slot * Hv + hv) * DK + 4 * part) * dv + j;
-  const bool fresh = seq_lens[r] == n, wide = (dv & 1) == 0;
+  const bool fresh = seq_lens[r] == n, wide = (dv & 1) == 0 && ((uintptr_t)rec_pool & 7) == 0;
   if (fresh || !act0) {
 #pragma unroll
     for (int x = 0; x < 16; ++x) S[0][x] = S[1][x] = 0ull;
@@ -632,11 +632,15 @@ __global__ void __launch_bounds__(256, 2) delta_step_kernel(const StepParams p) 
   }
 }
 
+// The step kernel (and the chunks) read states in pieces of 16 bytes and the convolution's weights in pieces of 8.
+static bool step_takes(int dk, int dv, int R, const void* w, const void* rec) {
+  return dk == 128 && dv == 128 && R <= 65535 && !((uintptr_t)w & 7) && !((uintptr_t)rec & 15);
+}
+
 // 0: the step kernel took every request; 1: those of one token (or none), the others are still to be done; < 0: error
 template <bool KDA>
 static int launch_step(StepParams p, int dk, int dv, cudaStream_t stream) {
-  // (the convolution's weights are read in pieces of 8 bytes)
-  if (dk != 128 || dv != 128 || p.R > 65535 || (!KDA && ((uintptr_t)p.w & 7))) return 1;
+  if (!step_takes(dk, dv, p.R, p.w, p.rec)) return 1;
   // no more tokens than requests: a step of single tokens (should one have more, its tokens go one after the other).  Else
   // single tokens beside prompts: the chunks of the prompt kernels would be nearly empty for them.
   p.single = p.T > p.R;
@@ -679,7 +683,7 @@ extern "C" int b200_gdn_forward(const void* mixed, int ldx, const void* a, const
   sp.R = R; sp.T = T; sp.Hk = Hk; sp.Hv = Hv; sp.ldx = ldx; sp.lda = lda;
   int rc = launch_step<false>(sp, dk, dv, stream);
   if (rc <= 0) return rc;
-  const int skip = dk == 128 && dv == 128 && R <= 65535 && !((uintptr_t)conv_w & 7);
+  const int skip = step_takes(dk, dv, R, conv_w, rec_pool);
   if (conv_out == nullptr || (chunks != nullptr ? !skip : (qn == nullptr || kn == nullptr || g == nullptr || beta == nullptr))) {
     b200_set_last_error("gdn_forward: scratch is missing", __FILE__, __LINE__);
     return -1;
@@ -769,7 +773,7 @@ extern "C" int b200_kda_forward(const void* q, const void* k, const void* v, int
   sp.R = R; sp.T = T; sp.Hk = Hk; sp.Hv = Hv; sp.ldq = ldq; sp.ldk = ldk; sp.ldv = ldv; sp.lower_bound = lower_bound;
   const int rc = launch_step<true>(sp, dk, dv, stream);
   if (rc <= 0) return rc;
-  const int skip = dk == 128 && dv == 128 && R <= 65535;
+  const int skip = step_takes(dk, dv, R, nullptr, rec_pool);
   const long long work = (long long)T * Hv * dk > (long long)T * Hk * 32 ? (long long)T * Hv * dk
                                                                          : (long long)T * Hk * 32;
   B200_CUDA_CHECK(launch_pdl(kda_prep_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), (size_t)0, stream,

@@ -22,7 +22,8 @@ def gdn_forward(mixed, a, b, meta, conv_pool, rec_pool, conv_w, A_log, dt_bias, 
         return torch.empty(shape, dtype=dtype, device=dev)
     out = new(T, Hv, dv, dtype=torch.bfloat16)
     conv_out = qn = kn = g = beta = chunks = None
-    step = dk == dv == 128 and conv_w.data_ptr() % 8 == 0           # single tokens have their own kernel
+    # single tokens have their own kernel, which reads weights in pieces of 8 bytes and states in pieces of 16
+    step = dk == dv == 128 and conv_w.data_ptr() % 8 == 0 and rec_pool.data_ptr() % 16 == 0
     if not step or T > R:
         conv_out = new(T, C, dtype=torch.bfloat16)
         # Chunks of 64 tokens on the tensor cores, or token by token: a token costs about 0.7 us there, a request's chunk
