@@ -46,6 +46,21 @@ def test_sources_do_not_name_closed_calls_or_cluster_multicast_loads():
         assert not multicast.search(text), p
 
 
+def test_arrivals_on_another_ctas_barrier_order_memory_at_cluster_scope():
+    """An arrival without a scope releases at CTA scope, which orders nothing for the threads of another CTA of the cluster."""
+    arrive = re.compile(r"mbarrier\.arrive[a-z_.:0-9]*")
+    for p in _sources():
+        if not p.endswith((".cu", ".cuh", ".h")):
+            continue
+        text = open(p).read()
+        for m in arrive.finditer(text):
+            if ".shared::cluster" not in m.group():
+                continue
+            before = text[max(0, m.start() - 120):m.start()]
+            assert ".release.cluster" in m.group() or (
+                ".relaxed.cluster" in m.group() and re.search(r"fence\.(release[a-z_:.]*|acq_rel)\.cluster", before)), (p, m.group())
+
+
 def test_built_artifacts_are_not_tracked():
     import subprocess
     r = subprocess.run(["git", "ls-files"], cwd=ROOT, capture_output=True, text=True)

@@ -22,7 +22,7 @@
 // Measured on B200 (CUDA events), 128 heads, mma.sync kernel -> this one: 4 x 2048 prompt tokens 32.5 -> 2.23 ms (71.9 -> 1050
 // TFLOP/s), 64 requests of 0.9 to 2 K keys 567 -> 61 us.  A chunk takes about 4500 cycles where its products need 2176:
 // K and V arrive late.  What mattered on the way: one elected thread issues (44 -> 32 cycles per product of N = 128),
-// arrivals on the leader's barriers release at CTA scope (at cluster scope each waits for the thread's stores, 700 cycles),
+// the one arrival a chunk on the leader's barrier releases shared memory at cluster scope (all memory: 2.22 -> 2.73 ms),
 // K and V have a copying warp each with the table entries fetched ahead.
 //
 // Semantics of the reference's dense MLA kernels (reference: src/vllm_torchtpu/kernels/mla/v2/).
@@ -131,8 +131,25 @@ __device__ __forceinline__ void load_boxes(uint8_t* dst, const CUtensorMap* m, u
       "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(0), "r"(panel), "r"(group)
       : "memory");
 }
+// The leader's product reads what this thread's warp stored to its own CTA's shared memory: the release has cluster scope,
+// and covers shared memory only (one that covers all memory waits about 1000 cycles for the way to L2).
 __device__ __forceinline__ void arrive_leader(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapa_shared(smem_u32(bar), 0)) : "memory");
+  asm volatile(
+      "fence.release.sync_restrict::shared::cta.cluster;\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa_shared(smem_u32(bar), 0))
+      : "memory");
+}
+// mbar_wait (which acquires at CTA scope) for what threads of the other CTA did before they arrived
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (!mbar_wait(bar, parity, abort_flag, status, code)) return false;
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\tselp.b32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t* r) {
   asm volatile(
@@ -169,10 +186,10 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SMEM_BAR);
   // in the leader only: both CTAs' copies or warps arrive there
-  uint64_t *q_full = bars, *k_full = bars + 1, *v_full = bars + 4, *s_empty = bars + 6, *p_full = bars + 8, *o_empty = bars + 9;
+  uint64_t *q_full = bars, *k_full = bars + 1, *v_full = bars + 4, *p_full = bars + 6;
   // in each CTA: the leader's commits arrive on both
-  uint64_t *q_empty = bars + 10, *k_empty = bars + 11, *v_empty = bars + 14, *s_full = bars + 16, *p_empty = bars + 18;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t *q_empty = bars + 7, *k_empty = bars + 8, *v_empty = bars + 11, *s_full = bars + 13, *p_empty = bars + 15;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank(), pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -185,10 +202,8 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 16);
     }
     mbar_init(p_full, 16);
-    mbar_init(o_empty, 16);
     mbar_init(p_empty, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -302,7 +317,6 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (elect_one()) {
           auto scores = [&](int j) -> bool {
             const int cc = c + j, b = cc & 1;
-            if (!mbar_wait(&s_empty[b], ((cc >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
             for (int g = 0; g < 3; ++g) {
               if (!mbar_wait(&k_full[g], cc & 1, abort_flag, p.status, ST_TIMEOUT_FULL)) return false;
               tc_fence_after();
@@ -322,8 +336,8 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           for (int j = 0; j < it.n && ok; ++j) {
             if (j + 1 < it.n && !(ok = scores(j + 1))) break;
             const int cc = c + j;
-            if (j == 0 && !(ok = mbar_wait(o_empty, (nq & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_TMEM_EMPTY))) break;
-            if (!(ok = mbar_wait(p_full, cc & 1, abort_flag, p.status, ST_TIMEOUT_FULL))) break;
+            // P is there, the scores that it is made of have been read and so has the output of the item before
+            if (!(ok = wait_cluster(p_full, cc & 1, abort_flag, p.status, ST_TIMEOUT_FULL))) break;
             for (int h = 0; h < 2 && ok; ++h) {
               if (!(ok = mbar_wait(&v_full[h], cc & 1, abort_flag, p.status, ST_TIMEOUT_FULL))) break;
               tc_fence_after();
@@ -365,9 +379,6 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         uint32_t s[32];
         tmem_ld_32x32(tmem + lane_addr + b * 64 + sh * 32, s);
         tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) arrive_leader(&s_empty[b]);    // the scores are in registers
         const int seen = lim - ((it.lo + j) * BK + part * 32) + 1;       // visible keys among these 32
         if (seen < 32) {
 #pragma unroll
@@ -417,13 +428,13 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             tmem_st_32x32(a + 32, o + 32);
           }
           tmem_st_wait();
-          tc_fence_before();
         }
 #pragma unroll
         for (int x = 0; x < 4; ++x)
           *reinterpret_cast<uint4*>(p_row + (((sh * 4 + x) ^ (r & 7)) << 4)) =
               make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
         fence_proxy_async_smem();
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive_leader(p_full);
       }
@@ -445,11 +456,6 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           tmem_ld_32x32(tmem + lane_addr + TM_O + sh * 128 + x, o);
           tmem_ld_32x32(tmem + lane_addr + TM_O + sh * 128 + x + 32, o + 32);
           tmem_ld_wait();
-          if (x == 64) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) arrive_leader(o_empty);
-          }
           if (!ok || !row_ok) continue;
           if (p.splits > 1) {
             float* d = p.part + ((size_t)it.split * p.T * p.H + row) * L + col + x;
