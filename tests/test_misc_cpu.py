@@ -265,3 +265,29 @@ def test_aux_files_of_a_uri_model_are_pulled_once_per_host(tmp_path):
     (src / "config.json").unlink()
     with pytest.raises(FileNotFoundError):
         ms.ensure_local_aux_files(f"file://{src}", str(tmp_path / "cache2"))
+
+
+def test_second_kernel_library_of_a_process_uses_its_own_symbols(tmp_path):
+    """A family's library loaded behind the full one: its errors are its own, so are the functions that it calls."""
+    import shutil
+    import subprocess
+    import sys
+
+    from vllm_torchtpu_b200.csrc import build
+    if not os.path.exists(build.lib_path()):
+        pytest.skip("kernel library not built")
+    other = str(tmp_path / "libb200_other.so")
+    shutil.copyfile(build.lib_path(), other)
+    code = f"""
+import ctypes
+from vllm_torchtpu_b200.csrc import build
+from vllm_torchtpu_b200.ops import cuda
+cuda.load_lib(build.lib_path())
+cuda.load_lib({other!r})
+n, one = ctypes.c_void_p(0), ctypes.c_int(1)
+rc = cuda.lib().b200_short_conv(n, one, n, n, n, n, n, n, one, one, one, ctypes.c_int(3), n)
+assert rc == -1 and b"short_conv" in cuda.lib().b200_get_last_error(), cuda.lib().b200_get_last_error()
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr

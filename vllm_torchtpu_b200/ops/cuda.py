@@ -71,9 +71,11 @@ def reload_lib(path: Optional[str] = None) -> str:
 
 
 def load_lib(path: str) -> None:
-    """Load this kernel library: the full one, or one that holds the sources of a model family only."""
+    """Load this kernel library: the full one, or one that holds the sources of a model family only.  Behind another
+    library it binds to its own symbols: kernels launched through the other one's stubs would run its code with this
+    one's state (and, where the sources differ, this one's arguments)."""
     global _lib, _sms
-    _lib = ctypes.CDLL(path, mode=ctypes.RTLD_GLOBAL)
+    _lib = ctypes.CDLL(path, mode=ctypes.RTLD_GLOBAL if _lib is None else os.RTLD_LOCAL | os.RTLD_DEEPBIND)
     _lib.b200_get_last_error.restype = ctypes.c_char_p
     for name in ("b200_attn_decode_scratch_bytes", "b200_linear_attention_chunk_bytes"):
         if hasattr(_lib, name):
