@@ -164,6 +164,57 @@ def test_attention_window_softcap_sinks():
     _attn_case([1, 130], [500, 300], 8, 2, 128, sinks=True, num_decode=1)
 
 
+def _one_request_each(q, kv, lens, bs=16):
+    """Prompt metadata and pages [blocks, 2, Hkv, bs, D] of requests whose keys and values kv [2, Hkv, sum of keys, D] holds."""
+    need = [-(-s // bs) for _, s in lens]
+    pages = torch.zeros(sum(need) + 1, 2, kv.shape[1], bs, kv.shape[3], dtype=kv.dtype, device=DEV)
+    bt = torch.zeros(len(lens), max(need), dtype=torch.int32, device=DEV)
+    at, off = 1, 0
+    for r, (_, s) in enumerate(lens):
+        bt[r, :need[r]] = torch.arange(at, at + need[r], device=DEV)
+        rows = torch.zeros(2, kv.shape[1], need[r] * bs, kv.shape[3], dtype=kv.dtype, device=DEV)
+        rows[:, :, :s] = kv[:, :, off:off + s]
+        pages[at:at + need[r]] = rows.view(2, kv.shape[1], need[r], bs, -1).permute(2, 0, 1, 3, 4)
+        at, off = at + need[r], off + s
+    qsl = torch.tensor([0] + [n for n, _ in lens], dtype=torch.int32).cumsum(0, dtype=torch.int32)
+    sl = torch.tensor([s for _, s in lens], dtype=torch.int32)
+    return pages, AttentionMetadata(
+        positions=None, slot_mapping=None, block_tables=bt, seq_lens=sl.to(DEV), query_start_loc=qsl.to(DEV), num_reqs=len(lens),
+        num_tokens=int(qsl[-1]), num_decode_reqs=0, max_query_len=max(n for n, _ in lens), max_seq_len=int(sl.max()),
+        padded_num_reqs=len(lens), padded_num_tokens=int(qsl[-1]), query_start_loc_cpu=qsl.long(), seq_lens_cpu=sl.long())
+
+
+def test_soft_cap_of_the_prompt_kernel():
+    """A row's largest score has weight one exactly: where a row sees one key the log-sum-exp is its capped score to the bit,
+    as fp32 gives it.  And outputs against 64 bits."""
+    g = torch.Generator(device=DEV).manual_seed(11)
+    Hq, Hkv, D, R, cap, scale = 32, 8, 128, 60, 50.0, 128 ** -0.5
+    q, kv = torch.zeros(R, Hq, D, device=DEV), torch.zeros(2, Hkv, R, D, device=DEV)
+    q[:, :, 0] = torch.randn(R, Hq, device=DEV, generator=g) * 40
+    kv[0, :, :, 0] = torch.randn(Hkv, R, device=DEV, generator=g) * 16
+    q, kv = q.bfloat16(), kv.bfloat16()
+    pages, meta = _one_request_each(q, kv, [(1, 1)] * R)
+    _, lse = cu().paged_attention(q, pages, meta, scale, softcap=cap, return_lse=True)
+    s = q[:, :, 0].float() * kv[0, :, :, 0].float().t().repeat_interleave(Hq // Hkv, 1)              # exact in fp32
+    log2e = torch.tensor(1.4426950408889634, device=DEV)
+    c = cap * log2e
+    want = c * torch.tanh(s * (torch.tensor(scale, device=DEV) * log2e) / c) * torch.tensor(0.6931471805599453, device=DEV)
+    assert (lse == want).float().mean() > 0.97, (lse == want).float().mean()
+    torch.testing.assert_close(lse, want, rtol=3e-7, atol=1e-7)
+
+    n, m = 200, 1100
+    q = torch.randn(n, Hq, D, device=DEV, generator=g).bfloat16()
+    kv = (torch.randn(2, Hkv, m, D, device=DEV, generator=g) * 4).bfloat16()
+    pages, meta = _one_request_each(q, kv, [(n, m)])
+    out = cu().paged_attention(q, pages, meta, scale, softcap=cap)
+    k, v = (t.double().repeat_interleave(Hq // Hkv, 0) for t in kv)
+    a = cap * torch.tanh(q.double().transpose(0, 1) @ k.transpose(1, 2) * scale / cap)
+    a = a.masked_fill(torch.ones(n, m, dtype=torch.bool, device=DEV).triu(m - n + 1), -float("inf"))
+    want = (torch.softmax(a, -1) @ v).transpose(0, 1)
+    # bf16 probabilities and outputs: 2^-9 each, uniform rounding, so about 2^-9 in the norm
+    assert (out.double() - want).norm() / want.norm() < 2 ** -8
+
+
 def test_argmax_and_sampling():
     R, V = 9, 128256
     g = torch.Generator(device=DEV).manual_seed(3)
