@@ -125,6 +125,13 @@ __device__ __forceinline__ Tile find_tile(const Params& p, int w, int total, int
   return t;
 }
 
+// The item of round k for this CTA: rounds go back and forth, so that who had the longest item of one round has the shortest
+// of the next (in one direction the first CTAs had the longest of all: 1000
+// tokens behind 500, 32 / 8 heads, soft cap, 238 us against 185; 8 x 1024 tokens 185 against 181).
+__device__ __forceinline__ int item_of(int k) {
+  return k * (int)gridDim.x + (k & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+}
+
 // FIN: the epilogue goes on to what p.fin describes.  CAP: scores are capped; the 64 hyperbolic tangents of a thread are
 // taken in two rounds on scores read once more (unrolled over registers they outgrow the instruction cache: 1000 tokens
 // behind 500, 32 / 8 heads, 290 us against 238).
@@ -191,7 +198,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // One chunk = 8 pages of K and 8 of V.  Lane l < 8 owns page l and issues its copies.
     int c = 0, nq = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+    for (int k = 0, w; (w = item_of(k)) < items && ok; ++k) {
       const Tile t = find_tile(p, w, total, lane);
       if (t.n == 0) continue;
       const int qb = nq & 1;
@@ -252,19 +259,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const uint32_t idesc_pv = umma_idesc_bf16_bmn(BM, D) & ~(p.pv_half ? (1u << 7) | (1u << 10) : 0u);
     const uint32_t q_addr = smem_u32(smem + SMEM_Q);
     const uint32_t p_addr = smem_u32(smem + SMEM_P);
-    // chunks of the next tile that has any, from item w on (0: none)
-    auto next_tile = [&](int& w) -> int {
-      for (; w < items; w += gridDim.x) {
+    // chunks of the next tile that has any, from round k on (0: none)
+    auto next_tile = [&](int& k) -> int {
+      for (int w; (w = item_of(k)) < items; ++k) {
         const int n = find_tile(p, w, total, lane).n;
         if (n > 0) return n;
       }
       return 0;
     };
-    int w = blockIdx.x, c = 0, nq = 0, n = next_tile(w);
+    int k = 0, c = 0, nq = 0, n = next_tile(k);
     bool ok = true, first = true;
     while (n > 0 && ok) {
-      w += gridDim.x;
-      const int n_next = next_tile(w);
+      ++k;
+      const int n_next = next_tile(k);
       if (elect_one()) {
         // scores of chunk cc with the queries of tile qi
         auto issue_qk = [&](int cc, int qi, bool begin, bool last) -> bool {
@@ -348,7 +355,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     };
     bool ok = true;
     int c = 0;
-    for (int w = blockIdx.x; w < items; w += gridDim.x) {
+    for (int k = 0, w; (w = item_of(k)) < items; ++k) {
       const Tile t = find_tile(p, w, total, lane);
       const int h = t.h, qs = t.qs, q0 = t.q0, nchunks = t.n, kv_end = t.kv_end;
       const int pos_local = row / p.G, head = h * p.G + row % p.G;
@@ -378,7 +385,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // sequence, sliding window); most chunks are fully visible
         const int c_hi = min(HC, min(lim, kv_end - 1) - tok0 + 1);
         const int c_lo = max(0, first - tok0);
-        if (c_lo > 0 || c_hi < HC) {
+        const bool cut = c_lo > 0 || c_hi < HC;
+        if (cut) {
 #pragma unroll
           for (int i = 0; i < HC; ++i)
             if (i < c_lo || i >= c_hi) sc[i] = 0xff800000u;
@@ -421,18 +429,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll 1
           for (int c0 = 0; c0 < HC; c0 += 32) {
             uint32_t rv[32], pk[16];
+            float e[32];
             tmem_ld_32x32(tmem_base + st * BKV + half * HC + lane_addr + c0, rv);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              float e[2];
+            for (int i = 0; i < 32; ++i) e[i] = ex2f(p.softcap * tanhf(__uint_as_float(rv[i]) * p.scale_log2 / p.softcap) - base);
+            if (cut) {
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                e[u] = ex2f(p.softcap * tanhf(__uint_as_float(rv[i + u]) * p.scale_log2 / p.softcap) - base);
-                if (c0 + i + u < c_lo || c0 + i + u >= c_hi) e[u] = 0.f;
-              }
-              pk[i >> 1] = pack(e[0], e[1]);
+              for (int i = 0; i < 32; ++i)
+                if (c0 + i < c_lo || c0 + i >= c_hi) e[i] = 0.f;
             }
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) pk[i >> 1] = pack(e[i], e[i + 1]);
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) put((c0 >> 3) + cc, pk + 4 * cc);
           }
