@@ -158,13 +158,30 @@ def test_attention_fp8_kv_cache_expanded_for_prompts(Hq, Hkv, bs, kw):
     _attn_case([3, 700], [1532, 0], Hq, Hkv, 128, num_decode=0, kv_fp8=True, scales=(1.0, 1.0), bs=bs, **kw)
 
 
+def test_expanded_pages_take_what_the_lengths_need(monkeypatch):
+    """One long request beside short ones: a pool of the pages of all of them, not of the longest for each."""
+    lens, bs, Hkv = [(300, 3000), (64, 64), (1, 17), (40, 1030)], 16, 8
+    g = torch.Generator(device=DEV).manual_seed(12)
+    kv = torch.randn(2, Hkv, sum(s for _, s in lens), 128, device=DEV, generator=g).to(torch.float8_e4m3fn).view(torch.uint8)
+    pages, meta = _one_request_each(kv, lens, bs)
+    pages = pages.view(torch.float8_e4m3fn)
+    q = torch.randn(meta.num_tokens, 32, 128, device=DEV, generator=g).bfloat16()
+    made, inner = [], cu()._expanded_pages
+    monkeypatch.setattr(cu(), "_expanded_pages", lambda *a: made.append(inner(*a)) or made[-1])
+    out = cu().paged_attention(q, pages, meta, 128 ** -0.5)
+    pool, table = made[0]
+    assert pool.shape[0] == sum(-(-s // bs) for _, s in lens) and table.shape[1] == -(-3000 // bs)
+    want = ref.paged_attention(q, pages, meta.block_tables, meta.seq_lens, meta.query_start_loc, 128 ** -0.5, num_reqs=len(lens))
+    _close(out, want, 2e-2, 2e-2)
+
+
 def test_attention_window_softcap_sinks():
     _attn_case([1, 130, 17], [500, 300, 0], 8, 2, 128, window=128, num_decode=1)
     _attn_case([1, 130], [500, 300], 8, 2, 128, softcap=30.0, num_decode=1)
     _attn_case([1, 130], [500, 300], 8, 2, 128, sinks=True, num_decode=1)
 
 
-def _one_request_each(q, kv, lens, bs=16):
+def _one_request_each(kv, lens, bs=16):
     """Prompt metadata and pages [blocks, 2, Hkv, bs, D] of requests whose keys and values kv [2, Hkv, sum of keys, D] holds."""
     need = [-(-s // bs) for _, s in lens]
     pages = torch.zeros(sum(need) + 1, 2, kv.shape[1], bs, kv.shape[3], dtype=kv.dtype, device=DEV)
@@ -193,7 +210,7 @@ def test_soft_cap_of_the_prompt_kernel():
     q[:, :, 0] = torch.randn(R, Hq, device=DEV, generator=g) * 40
     kv[0, :, :, 0] = torch.randn(Hkv, R, device=DEV, generator=g) * 16
     q, kv = q.bfloat16(), kv.bfloat16()
-    pages, meta = _one_request_each(q, kv, [(1, 1)] * R)
+    pages, meta = _one_request_each(kv, [(1, 1)] * R)
     _, lse = cu().paged_attention(q, pages, meta, scale, softcap=cap, return_lse=True)
     s = q[:, :, 0].float() * kv[0, :, :, 0].float().t().repeat_interleave(Hq // Hkv, 1)              # exact in fp32
     log2e = torch.tensor(1.4426950408889634, device=DEV)
@@ -205,7 +222,7 @@ def test_soft_cap_of_the_prompt_kernel():
     n, m = 200, 1100
     q = torch.randn(n, Hq, D, device=DEV, generator=g).bfloat16()
     kv = (torch.randn(2, Hkv, m, D, device=DEV, generator=g) * 4).bfloat16()
-    pages, meta = _one_request_each(q, kv, [(n, m)])
+    pages, meta = _one_request_each(kv, [(n, m)])
     out = cu().paged_attention(q, pages, meta, scale, softcap=cap)
     k, v = (t.double().repeat_interleave(Hq // Hkv, 0) for t in kv)
     a = cap * torch.tanh(q.double().transpose(0, 1) @ k.transpose(1, 2) * scale / cap)

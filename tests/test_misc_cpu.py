@@ -291,3 +291,41 @@ assert rc == -1 and b"short_conv" in cuda.lib().b200_get_last_error(), cuda.lib(
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
                        cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0, r.stderr
+
+
+def test_scratch_of_larger_steps_is_part_of_the_memory_budget(monkeypatch):
+    """The dummy run that sizes the KV cache has no context and few requests: what e4m3 prompts and the delta rule's chunks
+    take beyond it is added."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from vllm_torchtpu_b200.config import ModelConfig
+    from vllm_torchtpu_b200.platform import B200Platform
+    from vllm_torchtpu_b200.runner import model_runner as mr
+    dense = ModelConfig(num_q_heads=32, num_kv_heads=8, head_dim=128, max_model_len=4096)
+    hybrid = ModelConfig(architecture="qwen3_next", num_kv_heads=2, head_dim=256, gdn_num_k_heads=16, gdn_num_v_heads=32,
+                         gdn_head_k_dim=128, gdn_head_v_dim=128, max_model_len=4096)
+    e4m3 = torch.float8_e4m3fn
+    # 20 requests of 4096 tokens: 2 (key, value) * 8 heads * 128 * 2 bytes a token
+    assert mr.larger_step_scratch(dense, e4m3, 1, 8192, 20, 16) == 20 * 4096 * 4096
+    assert mr.larger_step_scratch(dense, e4m3, 2, 8192, 20, 16) == 20 * 4096 * 2048
+    assert mr.larger_step_scratch(dense, e4m3, 1, 8192, 256, 16) == 1 << 30
+    assert mr.larger_step_scratch(dense, torch.bfloat16, 1, 8192, 256, 16) == 0
+    assert mr.larger_step_scratch(hybrid, torch.bfloat16, 1, 8192, 64, 16) == 4 * (128 + 64) * 32 * (128 * 64 + 256)
+    assert mr.larger_step_scratch(hybrid, e4m3, 1, 8192, 64, 16) == 4 * (128 + 64) * 32 * (128 * 64 + 256)
+
+    seen = []
+    for name, value in (("synchronize", None), ("reset_peak_memory_stats", None), ("empty_cache", None),
+                        ("memory_allocated", 100), ("max_memory_allocated", 1100), ("mem_get_info", (1 << 40, 1 << 40))):
+        monkeypatch.setattr(torch.cuda, name, lambda value=value: value)
+    monkeypatch.setattr(B200Platform, "compute_hbm_budget", classmethod(
+        lambda cls, cfg, weights, peak: seen.append(peak) or SimpleNamespace(kv_cache=1 << 30)))
+    r = mr.ModelRunner.__new__(mr.ModelRunner)
+    r.cfg = SimpleNamespace(cache=SimpleNamespace(num_gpu_blocks_override=None, kv_cache_dtype="fp8", kv_cache_memory_bytes=None))
+    r.mcfg, r.block_size, r.extra_kv_layers, r.is_cuda, r.max_reqs, r.max_tokens = dense, 16, 0, True, 20, 8192
+    r.model = SimpleNamespace(kv_bytes_per_block=lambda bs, dt: 1 << 16, weight_bytes=lambda: 5)
+    monkeypatch.setattr(mr.ModelRunner, "init_kv_cache", lambda self, n: None)
+    monkeypatch.setattr(mr.ModelRunner, "_dummy_run", lambda self, t, n: None)
+    r.determine_num_blocks()
+    assert seen == [1000 + 20 * 4096 * 4096]

@@ -566,25 +566,43 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
 // Pages of an e4m3 cache expanded exactly, keys to bf16 (as the queries are), values to fp16 (so that the probabilities, of
 // the same type in one product, have 11 bits, as in the mma.sync kernel): 0.00167 from the result in 64 bits, 0.0022 with
-// bf16 values.  The pages of request nd + y at rows y * pages .. of the new pool; values behind the
-// sequence become zeros.  grid (pages, requests, 2 * Hkv); the block table of the new pool is written along.
+// bf16 values.  The pages of requests nd, nd + 1, .. lie one behind the other in the new pool; values behind a sequence
+// become zeros.  grid (total pages, 2 * Hkv); the block table of the new pool is written along.
 __global__ void __launch_bounds__(128) expand_pages_kernel(const uint8_t* __restrict__ kv, uint16_t* __restrict__ dst,
                                                            int* __restrict__ table, const int* __restrict__ block_tables,
-                                                           const int* __restrict__ seq_lens, int nd, int max_blocks,
+                                                           const int* __restrict__ seq_lens, int nd, int requests, int max_blocks,
                                                            int block_size, long long num_blocks, int H2, int pages) {
   pdl_launch_dependents();
   pdl_wait();
-  const int page = blockIdx.x, r = nd + blockIdx.y, seq = seq_lens[r];
-  if (page * block_size >= seq) return;
-  const int to = blockIdx.y * pages + page;
+  const int to = blockIdx.x, lane = threadIdx.x & 31;
+  int r = -1, page = to;
+  for (int b = 0; b < requests; b += 32) {
+    const int n = b + lane < requests ? (max(0, seq_lens[nd + b + lane]) + block_size - 1) / block_size : 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const int sum = __shfl_sync(0xffffffffu, incl, 31);
+    if (page < sum) {
+      const int first = __ffs(__ballot_sync(0xffffffffu, incl > page)) - 1;
+      r = nd + b + first;
+      page -= __shfl_sync(0xffffffffu, incl - n, first);
+      break;
+    }
+    page -= sum;
+  }
+  if (r < 0 || page >= pages) return;                 // (lengths are those that the host sized the pool for)
+  const int seq = seq_lens[r];
   long long blk = page < max_blocks ? block_tables[(size_t)r * max_blocks + page] : -1;
   if (blk < 0 || blk >= num_blocks) {
     B200_NOTE_BAD_INDEX();
     blk = 0;
   }
-  if (blockIdx.z == 0 && threadIdx.x == 0) table[(size_t)r * pages + page] = to;
-  const uint4* src = reinterpret_cast<const uint4*>(kv + ((size_t)blk * H2 + blockIdx.z) * block_size * D);
-  uint4* d = reinterpret_cast<uint4*>(dst + ((size_t)to * H2 + blockIdx.z) * block_size * D);
+  if (blockIdx.y == 0 && threadIdx.x == 0) table[(size_t)r * pages + page] = to;
+  const uint4* src = reinterpret_cast<const uint4*>(kv + ((size_t)blk * H2 + blockIdx.y) * block_size * D);
+  uint4* d = reinterpret_cast<uint4*>(dst + ((size_t)to * H2 + blockIdx.y) * block_size * D);
   const int rows = seq - page * block_size;
   for (int i = threadIdx.x; i < block_size * (D / 16); i += 128) {
     uint32_t o[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -596,7 +614,7 @@ __global__ void __launch_bounds__(128) expand_pages_kernel(const uint8_t* __rest
         uint32_t h;
         const uint16_t e = (uint16_t)(w[j >> 1] >> (16 * (j & 1)));
         asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"(e));
-        if (2 * blockIdx.z < H2) {
+        if (2 * blockIdx.y < H2) {
           const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
           const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
           o[j] = *reinterpret_cast<const uint32_t*>(&b);
@@ -688,19 +706,20 @@ extern "C" int b200_attn_prefill_tc(const void* q, const void* kv, void* out, fl
                               sinks, status, 0, stream, nullptr, ldo, pv_half);
 }
 
-// The pages of requests [nd, nd + requests) of an e4m3 cache [num_blocks, 2, Hkv, block_size, 128] expanded: dst [requests *
-// pages, 2, Hkv, block_size, 128], table [nd + requests, pages] (its first nd rows are left alone).
+// The pages of requests [nd, nd + requests) of an e4m3 cache [num_blocks, 2, Hkv, block_size, 128] expanded: dst [total, 2,
+// Hkv, block_size, 128] for the pages of all of them together, table [nd + requests, pages] for the most of one (its first nd
+// rows are left alone).
 extern "C" int b200_expand_e4m3_pages(const void* kv, void* dst, int* table, const int* block_tables, const int* seq_lens,
-                                      int nd, int requests, int pages, int max_blocks, int block_size, long long num_blocks,
-                                      int Hkv, cudaStream_t stream) {
-  if (requests <= 0 || pages <= 0) return 0;
-  if (requests > 65535 || 2 * Hkv > 65535 || (((uintptr_t)kv | (uintptr_t)dst) & 15)) {
-    b200_set_last_error("expand_e4m3_pages: at most 65535 requests, aligned pools", __FILE__, __LINE__);
+                                      int nd, int requests, int total, int pages, int max_blocks, int block_size,
+                                      long long num_blocks, int Hkv, cudaStream_t stream) {
+  if (requests <= 0 || total <= 0) return 0;
+  if (2 * Hkv > 65535 || (((uintptr_t)kv | (uintptr_t)dst) & 15)) {
+    b200_set_last_error("expand_e4m3_pages: aligned pools", __FILE__, __LINE__);
     return -1;
   }
-  B200_CUDA_CHECK(launch_pdl(fa::expand_pages_kernel, dim3(pages, requests, 2 * Hkv), dim3(128), (size_t)0, stream,
-                             (const uint8_t*)kv, (uint16_t*)dst, table, block_tables, seq_lens, nd, max_blocks, block_size,
-                             num_blocks, 2 * Hkv, pages));
+  B200_CUDA_CHECK(launch_pdl(fa::expand_pages_kernel, dim3(total, 2 * Hkv), dim3(128), (size_t)0, stream,
+                             (const uint8_t*)kv, (uint16_t*)dst, table, block_tables, seq_lens, nd, requests, max_blocks,
+                             block_size, num_blocks, 2 * Hkv, pages));
   return 0;
 }
 

@@ -708,25 +708,36 @@ def paged_attention(q, kv_cache, meta, scale, *, sliding_window=None, softcap=No
     return out
 
 
+EXPANDED_BYTES = 1 << 30              # most that a pool of expanded pages takes
+
+
+def expanded_scratch_bytes(max_reqs: int, max_len: int, block_size: int, Hkv: int, D: int) -> int:
+    """Most that a step's pool takes (``_expanded_pages``)."""
+    return min(EXPANDED_BYTES, max_reqs * -(-max_len // block_size) * 2 * Hkv * block_size * D * 2) if D == 128 else 0
+
+
 def _expanded_pages(kv_cache, meta, nd: int, R: int, heads_rows: int, window: int, v_scale: float):
     """Prompts over an e4m3 cache on the tcgen05 kernel, which reads 16-bit pages: the pages of requests nd .. R - 1
     expanded (exactly) into a pool of this call, with its block table.  None where the mma.sync kernel, which expands in
     registers, has to do it: lengths unknown to the host, a window (few of the pages would be read), a scale of the values
-    (it goes to the output there), pools above 1 GB; and where it is as fast, because the call is short and the second
-    launch and its tensors cost 15 us: 4.4 M (query head, key) pairs took 43 us there and 58 this way, 9.8 M 76 and 57."""
+    (it goes to the output there), pools above ``EXPANDED_BYTES``; and where it is as fast, because the call is short and the
+    second launch and its tensors cost 15 us: 4.4 M (query head, key) pairs took 43 us there and 58 this way, 9.8 M 76 and 57."""
     if (meta.seq_lens_cpu is None or window or v_scale != 1.0 or heads_rows * (meta.max_seq_len or 0) < 8_000_000
             or kv_cache.data_ptr() % 16 or torch.cuda.is_current_stream_capturing()):
         return None
     nb, _, Hkv, bs, D = kv_cache.shape
-    longest = int(meta.seq_lens_cpu[nd:R].max())
-    pages = -(-longest // bs)
-    if pages <= 0 or heads_rows * longest < 8_000_000 or bs % 16 or (R - nd) * pages * 2 * Hkv * bs * D > 1 << 29:
+    lens = meta.seq_lens_cpu.numpy()[nd:R]
+    if bs % 16 or heads_rows * int(lens.max()) < 8_000_000:
         return None
-    pool = torch.empty(((R - nd) * pages, 2, Hkv, bs, D), dtype=torch.bfloat16, device=kv_cache.device)
-    table = torch.empty((R, pages), dtype=torch.int32, device=kv_cache.device)
+    need = (lens + (bs - 1)) // bs
+    total, most = int(need.sum()), int(need.max())
+    if total <= 0 or total * 2 * Hkv * bs * D * 2 > EXPANDED_BYTES:
+        return None
+    pool = torch.empty((total, 2, Hkv, bs, D), dtype=torch.bfloat16, device=kv_cache.device)
+    table = torch.empty((R, most), dtype=torch.int32, device=kv_cache.device)
     _check(lib().b200_expand_e4m3_pages(
-        _p(kv_cache), _p(pool), _p(table), _p(meta.block_tables), _p(meta.seq_lens), c_int(nd), c_int(R - nd), c_int(pages),
-        c_int(meta.block_tables.shape[1]), c_int(bs), c_longlong(nb), c_int(Hkv), _stream()), "expand_e4m3_pages")
+        _p(kv_cache), _p(pool), _p(table), _p(meta.block_tables), _p(meta.seq_lens), c_int(nd), c_int(R - nd), c_int(total),
+        c_int(most), c_int(meta.block_tables.shape[1]), c_int(bs), c_longlong(nb), c_int(Hkv), _stream()), "expand_e4m3_pages")
     count_launch()
     return pool, table
 

@@ -10,6 +10,16 @@ from . import cuda as _c
 
 
 CHUNK_WORDS = 128 * 64 + 4 * 64           # scratch of a (chunk, head) in gdn_chunk.cu
+MOST_WORDS = 1 << 28                      # most that a call takes for them (1 GB)
+
+
+def chunk_words(T: int, R: int, Hv: int) -> int:
+    return (T // 64 + R) * Hv * CHUNK_WORDS
+
+
+def chunk_scratch_bytes(max_tokens: int, max_reqs: int, Hv: int) -> int:
+    """Most that ``gdn_forward`` takes for its chunks in a step."""
+    return 4 * min(MOST_WORDS, chunk_words(max_tokens, max_reqs, Hv))
 
 
 def gdn_forward(mixed, a, b, meta, conv_pool, rec_pool, conv_w, A_log, dt_bias, Hk, Hv, dk, dv):
@@ -27,10 +37,10 @@ def gdn_forward(mixed, a, b, meta, conv_pool, rec_pool, conv_w, A_log, dt_bias, 
     if not step or T > R:
         conv_out = new(T, C, dtype=torch.bfloat16)
         # Chunks of 64 tokens on the tensor cores, or token by token: a token costs about 0.7 us there, a request's chunk
-        # about 8 us with the work in front of it.  A wrong length costs time only.  (Scratch of at most 1 GB: 0.5 KB a token and head.)
+        # about 8 us with the work in front of it.  A wrong length costs time only.
         longest = meta.max_query_len if meta.max_query_len > 1 else T - R + 1
-        words = (T // 64 + R) * Hv * CHUNK_WORDS
-        if step and longest > 16 and words <= 1 << 28:
+        words = chunk_words(T, R, Hv)
+        if step and longest > 16 and words <= MOST_WORDS:
             chunks = new(words)
         else:
             qn, kn, g, beta = new(T, Hk, dk), new(T, Hk, dk), new(T, Hv), new(T, Hv)

@@ -136,6 +136,18 @@ class StepResult:
         return out
 
 
+def larger_step_scratch(mc, kv_dtype, tp: int, max_tokens: int, max_reqs: int, block_size: int) -> int:
+    """Bytes that a step's kernels may take beyond what the dummy run shows, which has no context and few requests: scratch
+    that grows with either.  Layers run one after the other, so the largest one counts."""
+    from ..ops import cuda, cuda_gdn
+    got = 0
+    if kv_dtype == torch.float8_e4m3fn and not mc.is_mla:
+        got = cuda.expanded_scratch_bytes(max_reqs, mc.max_model_len, block_size, max(1, mc.num_kv_heads // tp), mc.head_dim)
+    if mc.architecture == "qwen3_next" and mc.gdn_head_k_dim == mc.gdn_head_v_dim == 128:
+        got = max(got, cuda_gdn.chunk_scratch_bytes(max_tokens, max_reqs, mc.gdn_num_v_heads // tp))
+    return got
+
+
 class ModelRunner:
     def __init__(self, cfg: EngineConfig, device: Optional[str] = None):
         self.cfg = cfg
@@ -269,6 +281,7 @@ class ModelRunner:
         self._dummy_run(self.max_tokens, min(self.max_reqs, max(1, self.max_tokens // 128)))
         torch.cuda.synchronize()
         peak = torch.cuda.max_memory_allocated() - base
+        peak += larger_step_scratch(self.mcfg, kv_dtype, get_state().tp.size, self.max_tokens, self.max_reqs, self.block_size)
         self.kv_caches = []
         torch.cuda.empty_cache()
         budget = B200Platform.compute_hbm_budget(self.cfg, self.model.weight_bytes(), peak)
