@@ -329,3 +329,19 @@ def test_scratch_of_larger_steps_is_part_of_the_memory_budget(monkeypatch):
     monkeypatch.setattr(mr.ModelRunner, "_dummy_run", lambda self, t, n: None)
     r.determine_num_blocks()
     assert seen == [1000 + 20 * 4096 * 4096]
+
+
+# (tokens, keys) of the requests, heads; measured us on mma.sync and on expanded pages
+@pytest.mark.parametrize("shape,Hq,Hkv,pays", [
+    ([(16, 1100)] * 64, 8, 8, False),                      # 153, 197
+    ([(32, 1032)] * 128, 8, 8, False),                     # 223, 330
+    ([(128, 128)] * 8, 64, 8, False),                      # 32, 44
+    ([(64, 64)], 32, 8, False),                            # 21, 43
+    ([(16, 1100)] * 64, 32, 8, True),                      # 427, 200
+    ([(64, 32064)] * 2, 8, 8, True),                       # 1535, 544: the longest chain, not the sum
+    ([(677, 1701)] * 3, 32, 8, True), ([(2000, 2000)], 16, 8, True),
+    ([(64, 16000)] + [(64, 64)] * 31, 32, 8, True)])
+def test_rule_for_expanded_pages(shape, Hq, Hkv, pays):
+    from vllm_torchtpu_b200.ops.cuda import expansion_pays
+    work = Hq * sum(-(-q // 64) * n for q, n in shape)
+    assert expansion_pays(work, sum(n for _, n in shape), max(n for _, n in shape), Hkv) is pays

@@ -668,9 +668,11 @@ def paged_attention(q, kv_cache, meta, scale, *, sliding_window=None, softcap=No
         nd = 0
     if R > nd:
         qsl = meta.query_start_loc_cpu
+        q_tiles = None
         if qsl is not None:
-            ql = (qsl[nd + 1:R + 1] - qsl[nd:R])
-            tiles = int(((ql + 63) // 64).sum())
+            ql = qsl.numpy()
+            q_tiles = (ql[nd + 1:R + 1] - ql[nd:R] + 63) // 64
+            tiles = int(q_tiles.sum())
         else:
             tiles = (T + 63) // 64 + (R - nd)
         if meta.dcp_size > 1:
@@ -684,7 +686,7 @@ def paged_attention(q, kv_cache, meta, scale, *, sliding_window=None, softcap=No
                 c_float(cap), c_int(meta.dcp_size), c_int(meta.dcp_rank), c_int(meta.dcp_interleave), _stream()),
                 "attn_prefill_dcp")
         elif (D == 128 and G in (1, 2, 4, 8) and envs.B200_ATTN_PREFILL_IMPL == "tc"
-              and (not kv_fp8 or (wide := _expanded_pages(kv_cache, meta, nd, R, (T - nd) * Hq, window, v_scale)) is not None)):
+              and (not kv_fp8 or (wide := _expanded_pages(kv_cache, meta, nd, R, q_tiles, tiles, Hq, window, v_scale)) is not None)):
             # tcgen05 kernel: 128 / G positions of a kv head per tile, K/V shared by the GQA group
             pool, table = wide if kv_fp8 else (kv_cache, meta.block_tables)
             _check(L.b200_attn_prefill_tc(
@@ -716,22 +718,33 @@ def expanded_scratch_bytes(max_reqs: int, max_len: int, block_size: int, Hkv: in
     return min(EXPANDED_BYTES, max_reqs * -(-max_len // block_size) * 2 * Hkv * block_size * D * 2) if D == 128 else 0
 
 
-def _expanded_pages(kv_cache, meta, nd: int, R: int, heads_rows: int, window: int, v_scale: float):
+def expansion_pays(work: int, keys: int, longest: int, Hkv: int) -> bool:
+    """Whether prompts are faster on expanded pages: ``work`` = sum over requests and query heads of (tiles of 64 tokens x
+    keys), ``keys`` of all requests, ``longest`` of one.  Estimates in us that 499 measured shapes gave (2 to 2000 tokens, 1
+    to 128 requests, 0 to 32 K keys in front, 1 to 8 query heads per kv head): the mma.sync kernel takes 0.18 ns a unit
+    of work, or 50 ns per key of its longest chain; the expansion 22 us with its launch and tensors and 0.15 ns per key
+    and kv head, the tcgen05 kernel 0.03 ns a unit of work, or 16 ns per key of its longest.  The faster way but for 0.5 %
+    in the mean, and no shape more than 8 % slower than on mma.sync.  (A bound on (query head, key) pairs alone: 10 % in
+    the mean; 64 x 16 tokens with 1100 keys, 8 / 8 heads, 153 us on mma.sync, 197 expanded.)"""
+    return (max(0.18 * work, 50 * longest) > 22_000 + 0.15 * Hkv * keys + max(0.03 * work, 16 * longest))
+
+
+def _expanded_pages(kv_cache, meta, nd: int, R: int, q_tiles, tiles: int, Hq: int, window: int, v_scale: float):
     """Prompts over an e4m3 cache on the tcgen05 kernel, which reads 16-bit pages: the pages of requests nd .. R - 1
     expanded (exactly) into a pool of this call, with its block table.  None where the mma.sync kernel, which expands in
     registers, has to do it: lengths unknown to the host, a window (few of the pages would be read), a scale of the values
-    (it goes to the output there), pools above ``EXPANDED_BYTES``; and where it is as fast, because the call is short and the
-    second launch and its tensors cost 15 us: 4.4 M (query head, key) pairs took 43 us there and 58 this way, 9.8 M 76 and 57."""
-    if (meta.seq_lens_cpu is None or window or v_scale != 1.0 or heads_rows * (meta.max_seq_len or 0) < 8_000_000
-            or kv_cache.data_ptr() % 16 or torch.cuda.is_current_stream_capturing()):
+    (it goes to the output there), pools above ``EXPANDED_BYTES``; and where it is as fast (``expansion_pays``)."""
+    longest = meta.max_seq_len or 0
+    if (meta.seq_lens_cpu is None or q_tiles is None or window or v_scale != 1.0 or kv_cache.data_ptr() % 16
+            or max(0.18 * tiles * Hq * longest, 50 * longest) <= 22_000 or torch.cuda.is_current_stream_capturing()):
         return None
     nb, _, Hkv, bs, D = kv_cache.shape
-    lens = meta.seq_lens_cpu.numpy()[nd:R]
-    if bs % 16 or heads_rows * int(lens.max()) < 8_000_000:
+    if bs % 16:
         return None
-    need = (lens + (bs - 1)) // bs
+    need = (meta.seq_lens_cpu.numpy()[nd:R] + (bs - 1)) // bs
     total, most = int(need.sum()), int(need.max())
-    if total <= 0 or total * 2 * Hkv * bs * D * 2 > EXPANDED_BYTES:
+    if (total <= 0 or total * 2 * Hkv * bs * D * 2 > EXPANDED_BYTES
+            or not expansion_pays(int(q_tiles.dot(need)) * bs * Hq, total * bs, most * bs, Hkv)):
         return None
     pool = torch.empty((total, 2, Hkv, bs, D), dtype=torch.bfloat16, device=kv_cache.device)
     table = torch.empty((R, most), dtype=torch.int32, device=kv_cache.device)
