@@ -301,6 +301,34 @@ def test_sampling_sizes_and_types(V, dtype):
     assert torch.equal(got.long(), want)
 
 
+# clusters of 8, 4, 2 and 1 CTA and their instances of 8, 16 and 32 keys a thread at their limits, rows beyond which a second
+# launch takes those of which nothing is cut
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("R,V", [(9, 8193), (10, 8193), (18, 65537), (37, 32768), (38, 8193), (74, 32769), (75, 16384), (150, 8193),
+                                 (400, 4097), (130, 32770), (150, 32770), (96, 163000), (64, 163000)])
+def test_sampling_of_many_rows_draws_what_few_rows_draw(R, V, dtype):
+    """A row's token depends on the row, not on how many there are: the first rows alone take clusters of eight."""
+    g = torch.Generator(device=DEV).manual_seed(R)
+    logits = (torch.randn(R, V, device=DEV, generator=g) * 2.0).to(dtype)
+    logits[1, 5:] = -float("inf")
+    temp = torch.rand(R, device=DEV, generator=g) + 0.3
+    temp[2] = 0.0
+    top_k = torch.tensor([0, 0, 0, 50, 600, 0, 1, V], device=DEV, dtype=torch.int32).repeat(R // 8 + 1)[:R].contiguous()
+    top_p = torch.tensor([1.0, 1.0, 0.5, 0.9, 1.0, 0.95, 1.0, 1.0], device=DEV).repeat(R // 8 + 1)[:R].contiguous()
+    step = torch.tensor([3], dtype=torch.int64, device=DEV)
+    draw = lambda n: cu().sample(logits[:n], temp[:n], top_k[:n], top_p[:n], seed=7, step_tensor=step)       # noqa: E731
+    many, few = draw(R), draw(8)
+    assert torch.equal(many[:8], few)
+    # noise made in front of the call is drawn from element by element
+    u = cu().philox_uniform(R, V, 7, 3, DEV)
+    assert torch.equal(many, cu().sample(logits, temp, top_k, top_p, uniform=u))
+    free = (((top_k <= 0) | (top_k >= V)) & (top_p >= 1) & (temp > 0)).nonzero()[:, 0]
+    x = logits.float() * (1.0 / temp.clamp_min(1e-5))[:, None] - torch.log(-torch.log(u.clamp(1e-20, 1.0 - 1e-7)))
+    # the kernel's logarithm has an absolute error of 2^-21 near one, where -log(u) of the winners is 1e-5: 0.05 of noise
+    got, best = x.gather(1, many.long()[:, None])[:, 0], x.amax(-1)
+    assert (best - got)[free].max() < 1.0
+
+
 def test_logprobs():
     R, V = 5, 32000
     logits = torch.randn(R, V, device=DEV).bfloat16()

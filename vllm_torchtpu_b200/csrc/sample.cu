@@ -145,13 +145,19 @@ argmax_kernel(const T* __restrict__ logits, int ld, int V, int* __restrict__ out
   if (threadIdx.x == 0) out[blockIdx.x] = a.i < V ? a.i : 0;
 }
 
+// rows that one pass settles: the arg-max, or a draw from all logits
+__device__ __forceinline__ bool nothing_cut(const float* temperature, const int* top_k, const float* top_p, int r, int V) {
+  return temperature[r] <= 1e-5f || ((top_k[r] <= 0 || top_k[r] >= V) && top_p[r] >= 1.f);
+}
+
 // Full sampler.  temperature <= 1e-5 -> greedy.  top_k <= 0 and top_p >= 1 disable the filters.
 template <typename T>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const T* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const float* __restrict__ uniform, unsigned long long seed, unsigned long long step,
-              const long long* __restrict__ step_ptr, int* __restrict__ out) {
+              const long long* __restrict__ step_ptr, int* __restrict__ out, int whole_only) {
+  if (whole_only && !nothing_cut(temperature, top_k, top_p, blockIdx.x, V)) return;
   if (step_ptr != nullptr) step += (unsigned long long)(*step_ptr);   // graph replays read a fresh offset
   __shared__ ArgMax red[32];
   __shared__ float redf[32];
@@ -236,14 +242,12 @@ sample_kernel(const T* __restrict__ logits, int ld, int V, const float* __restri
   if (threadIdx.x == 0) out[r] = a.i < V ? a.i : 0;
 }
 
-// ---- the same sampler with the row held in registers by a cluster of eight CTAs ------------------------
+// ---- the same sampler with the row held in registers by a cluster of CTAs ------------------------------
 // The single-CTA kernel above re-reads its row from L2 in every bisection pass (about 70 passes: 1.2 to 1.9 ms for rows
-// of 151936).  Here a cluster of SAMPLE_CL CTAs owns a row: CTA c keeps elements [c * seg, (c + 1) * seg) as 32-bit keys
+// of 151936).  Here a cluster of CL CTAs owns a row: CTA c keeps elements [c * seg, (c + 1) * seg) as 32-bit keys
 // in registers (NPT per thread), so a pass is NPT compares per thread, a block reduction and one exchange of a few
 // words over distributed shared memory.  The threshold searches are 4-ary (three thresholds per pass), which halves the
 // number of cluster barriers.  Same thresholds, same Philox noise and same Gumbel-max draw as the single-CTA kernel.
-// Eight CTAs, so that a thread has 32 keys of 128 K logits and two CTAs fit an SM.
-constexpr int SAMPLE_CL = 8;
 constexpr int SAMPLE_CT = 512;                    // threads per CTA of the cluster kernel
 constexpr int SAMPLE_LIST = 2048;                 // candidates of a row that the first CTA takes over
 
@@ -297,38 +301,42 @@ __device__ __forceinline__ void block_sum3_i(int& a, int& b, int& c, int* red) {
 }
 
 // Four words of every CTA's slot, one per lane (CTA = lane / 4), summed over the CTAs: lane w gets word w.
-template <typename V>
+template <int CL, typename V>
 __device__ __forceinline__ V lane_of_cluster(uint32_t slot) {
-  static_assert(SAMPLE_CL == 8, "a warp reads the slots of eight CTAs");
+  static_assert(CL <= 8, "a warp reads the slots of eight CTAs");
   const int lane = threadIdx.x & 31;
-  const uint32_t addr = mapa_shared(slot, lane >> 2) + 4 * (lane & 3);
+  const uint32_t addr = mapa_shared(slot, min(lane >> 2, CL - 1)) + 4 * (lane & 3);
   V v;
   if constexpr (sizeof(V) == 4 && V(0.5f) != V(0)) v = ld_dsmem_f32(addr); else v = ld_dsmem_s32(addr);
+  if ((lane >> 2) >= CL) v = 0;
   v += __shfl_xor_sync(0xffffffffu, v, 4);
   v += __shfl_xor_sync(0xffffffffu, v, 8);
   v += __shfl_xor_sync(0xffffffffu, v, 16);
   return v;
 }
 
+template <int CL>
 __device__ __forceinline__ void cluster_sum3_f(float& a, float& b, float& c, ClusterXchg* x, float* red, int& par) {
   block_sum3_f(a, b, c, red);
   if (threadIdx.x == 0) { x->f[par][0] = a; x->f[par][1] = b; x->f[par][2] = c; }
   cluster_arrive_release();
   cluster_wait_acquire();
-  float v = lane_of_cluster<float>(smem_u32(&x->f[par][0]));
+  float v = lane_of_cluster<CL, float>(smem_u32(&x->f[par][0]));
   a = __shfl_sync(0xffffffffu, v, 0); b = __shfl_sync(0xffffffffu, v, 1); c = __shfl_sync(0xffffffffu, v, 2);
   par ^= 1;
 }
+template <int CL>
 __device__ __forceinline__ void cluster_sum3_i(int& a, int& b, int& c, ClusterXchg* x, int* red, int& par) {
   block_sum3_i(a, b, c, red);
   if (threadIdx.x == 0) { x->i[par][0] = a; x->i[par][1] = b; x->i[par][2] = c; }
   cluster_arrive_release();
   cluster_wait_acquire();
-  int v = lane_of_cluster<int>(smem_u32(&x->i[par][0]));
+  int v = lane_of_cluster<CL, int>(smem_u32(&x->i[par][0]));
   a = __shfl_sync(0xffffffffu, v, 0); b = __shfl_sync(0xffffffffu, v, 1); c = __shfl_sync(0xffffffffu, v, 2);
   par ^= 1;
 }
 // cluster-wide arg-max of (value, index): smaller index wins ties
+template <int CL>
 __device__ __forceinline__ ArgMax cluster_argmax(ArgMax a, ClusterXchg* x, ArgMax* red, int& par) {
   a = block_argmax(a, red);
   if (threadIdx.x == 0) { x->f[par][3] = a.v; x->i[par][3] = a.i; }
@@ -337,7 +345,7 @@ __device__ __forceinline__ ArgMax cluster_argmax(ArgMax a, ClusterXchg* x, ArgMa
   const uint32_t bf = smem_u32(&x->f[par][3]), bi = smem_u32(&x->i[par][3]);
   ArgMax best{-INFINITY, 0x7fffffff};
 #pragma unroll
-  for (int r = 0; r < SAMPLE_CL; ++r) {
+  for (int r = 0; r < CL; ++r) {
     const ArgMax o{ld_dsmem_f32(mapa_shared(bf, r)), ld_dsmem_s32(mapa_shared(bi, r))};
     best = better(best, o);
   }
@@ -422,12 +430,13 @@ __device__ __forceinline__ void sample_list(const uint2* list, int n, int k, flo
 }
 
 // Element j of thread t is row index cr * seg + ((j >> 1) * 512 + t) * 2 + (j & 1).
-template <typename T, int SAMPLE_NPT>
+template <typename T, int SAMPLE_NPT, int CL>
 __global__ void __launch_bounds__(SAMPLE_CT, SAMPLE_NPT <= 32 ? 2 : 1)
 sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
                       const int* __restrict__ top_k, const float* __restrict__ top_p,
                       const float* __restrict__ uniform, unsigned long long seed, unsigned long long step,
-                      const long long* __restrict__ step_ptr, int* __restrict__ out) {
+                      const long long* __restrict__ step_ptr, int* __restrict__ out, int cut_only) {
+  if (cut_only && nothing_cut(temperature, top_k, top_p, blockIdx.x / CL, V)) return;      // (the whole cluster)
   if (step_ptr != nullptr) step += (unsigned long long)(*step_ptr);
   __shared__ ArgMax red[32];
   __shared__ float redf[96];
@@ -437,14 +446,14 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
   __shared__ unsigned long long red64[2][16];
   __shared__ uint32_t list_n, thread_max[SAMPLE_CT];
   if (threadIdx.x == 0) list_n = 0;
-  const int r = blockIdx.x / SAMPLE_CL;
+  const int r = blockIdx.x / CL;
   const int cr = (int)cluster_ctarank();
   const T* row = logits + (size_t)r * ld;
   const float temp = temperature[r];
   const bool greedy = temp <= 1e-5f;
   const float inv_t = greedy ? 1.f : 1.f / temp;
   // elements per CTA: a multiple of 2 * 512 so that pairs never straddle CTAs
-  const int seg = ((V + SAMPLE_CL - 1) / SAMPLE_CL + 2 * SAMPLE_CT - 1) / (2 * SAMPLE_CT) * (2 * SAMPLE_CT);
+  const int seg = ((V + CL - 1) / CL + 2 * SAMPLE_CT - 1) / (2 * SAMPLE_CT) * (2 * SAMPLE_CT);
   const int base = cr * seg + 2 * (int)threadIdx.x;
   int par = 0;
   // order-preserving 32-bit keys of the scaled logits; padding holds the key of -inf (KEY_NEG)
@@ -478,7 +487,7 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
       const float x = key2f(key[j]);
       if (x > a.v) a = ArgMax{x, idx(j)};
     }
-    a = cluster_argmax(a, &xchg, red, par);
+    a = cluster_argmax<CL>(a, &xchg, red, par);
     if (cr == 0 && threadIdx.x == 0) out[r] = a.i < V ? a.i : 0;
     cluster_arrive_release();                   // nobody leaves while a peer may still read its slots
     cluster_wait_acquire();
@@ -517,7 +526,7 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
     cluster_wait_acquire();
     uint32_t lowest = KEY_NEG + 1;                // (padding is never a candidate)
 #pragma unroll
-    for (int c = 0; c < SAMPLE_CL; ++c) lowest = max(lowest, (uint32_t)ld_dsmem_s32(mapa_shared(smem_u32(&xchg.i[par][0]), c)));
+    for (int c = 0; c < CL; ++c) lowest = max(lowest, (uint32_t)ld_dsmem_s32(mapa_shared(smem_u32(&xchg.i[par][0]), c)));
     par ^= 1;
     const uint32_t n_addr = mapa_shared(smem_u32(&list_n), 0), list_addr = mapa_shared(smem_u32(list), 0);
 #pragma unroll
@@ -553,7 +562,7 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
       for (int j = 0; j < SAMPLE_NPT; ++j) {
         c1 += key[j] >= u1; c2 += key[j] >= u2; c3 += key[j] >= u3;
       }
-      cluster_sum3_i(c1, c2, c3, &xchg, redi, par);
+      cluster_sum3_i<CL>(c1, c2, c3, &xchg, redi, par);
       if (t3 <= hi && c3 >= k) lo = t3;
       else if (t2 <= hi && c2 >= k) { lo = t2; hi = min(hi, t3 - 1); }
       else if (t1 <= hi && c1 >= k) { lo = t1; hi = min(hi, t2 - 1); }
@@ -571,14 +580,14 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
       if (x > m.v) m = ArgMax{x, idx(j)};
     }
   }
-  const float mx = cluster_argmax(m, &xchg, red, par).v;
+  const float mx = cluster_argmax<CL>(m, &xchg, red, par).v;
   uint32_t thr = kth;
   if (pp < 1.f) {
     float z = 0.f, z2 = 0.f, z3 = 0.f;
 #pragma unroll
     for (int j = 0; j < SAMPLE_NPT; ++j)
       if (key[j] >= kth) z += __expf(key2f(key[j]) - mx);
-    cluster_sum3_f(z, z2, z3, &xchg, redf, par);
+    cluster_sum3_f<CL>(z, z2, z3, &xchg, redf, par);
     // largest key such that mass(x >= key) >= top_p * Z (ties at the threshold are all kept)
     unsigned long long lo = kth, hi = f2key(mx);
     const float want = pp * z;
@@ -596,7 +605,7 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
           if (key[j] >= u3) m3 += e;
         }
       }
-      cluster_sum3_f(m1, m2, m3, &xchg, redf, par);
+      cluster_sum3_f<CL>(m1, m2, m3, &xchg, redf, par);
       if (t3 <= hi && m3 >= want) lo = t3;
       else if (t2 <= hi && m2 >= want) { lo = t2; hi = min(hi, t3 - 1); }
       else if (t1 <= hi && m1 >= want) { lo = t1; hi = min(hi, t2 - 1); }
@@ -606,17 +615,25 @@ sample_cluster_kernel(const T* __restrict__ logits, int ld, int V, const float* 
   }
   // ---- Gumbel-max over the kept set
   ArgMax a{-INFINITY, 0x7fffffff};
+  auto draw = [&](int j, float u) {
+    u = fminf(fmaxf(u, 1e-20f), 1.f - 1e-7f);
+    const float v = key2f(key[j]) - __logf(-__logf(u));
+    if (v > a.v || (v == a.v && idx(j) < a.i)) a = ArgMax{v, idx(j)};
+  };
+  if (thr == KEY_NEG + 1 && uniform == nullptr) {
+    // Nothing is cut: no branch an element, so that the noise of several is under way at a time.  (Padding and masked
+    // logits are -inf: they win nothing against the first element, which stands for none.)
+    a.i = -1;
 #pragma unroll
-  for (int j = 0; j < SAMPLE_NPT; ++j) {
-    const int i = idx(j);
-    if (key[j] >= thr) {
-      float u = uniform != nullptr ? uniform[(size_t)r * V + i] : uniform_at(seed, step, r, i);
-      u = fminf(fmaxf(u, 1e-20f), 1.f - 1e-7f);
-      const float v = key2f(key[j]) - __logf(-__logf(u));
-      if (v > a.v || (v == a.v && i < a.i)) a = ArgMax{v, i};
-    }
+    for (int j = 0; j < SAMPLE_NPT; ++j)
+      if ((j & ~3) / 2 * 2 * SAMPLE_CT < seg) draw(j, uniform_at(seed, step, r, idx(j)));
+    if (a.i < 0) a.i = 0x7fffffff;
+  } else {
+#pragma unroll
+    for (int j = 0; j < SAMPLE_NPT; ++j)
+      if (key[j] >= thr) draw(j, uniform != nullptr ? uniform[(size_t)r * V + idx(j)] : uniform_at(seed, step, r, idx(j)));
   }
-  a = cluster_argmax(a, &xchg, red, par);
+  a = cluster_argmax<CL>(a, &xchg, red, par);
   if (cr == 0 && threadIdx.x == 0) out[r] = a.i < V ? a.i : 0;
   cluster_arrive_release();
   cluster_wait_acquire();
@@ -887,43 +904,65 @@ extern "C" int b200_sample(const void* logits, int dtype, int R, int V, int ld, 
                            int* out, cudaStream_t stream) {
   if (R == 0) return 0;
   // below 4096 a row is one CTA's business; above 262144 the keys do not fit the registers of a cluster
-  if (V >= 4096 && V <= SAMPLE_CL * SAMPLE_CT * 64 && sample_cluster_enabled()) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(R * SAMPLE_CL);
-    cfg.blockDim = dim3(SAMPLE_CT);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = SAMPLE_CL;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    // the fewest keys per thread that hold the row: passes run over all of them
-#define SAMPLE_LAUNCH(T, NPT)                                                                                          \
-  B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, sample_cluster_kernel<T, NPT>, (const T*)logits, ld, V, temperature, top_k, \
-                                     top_p, uniform, seed, step, step_ptr, out))
-#define SAMPLE_SIZES(T)                                                   \
-  do {                                                                    \
-    if (V <= SAMPLE_CL * SAMPLE_CT * 8) SAMPLE_LAUNCH(T, 8);              \
-    else if (V <= SAMPLE_CL * SAMPLE_CT * 32) SAMPLE_LAUNCH(T, 32);       \
-    else if (V <= SAMPLE_CL * SAMPLE_CT * 40) SAMPLE_LAUNCH(T, 40);       \
-    else SAMPLE_LAUNCH(T, 64);                                            \
-  } while (0)
-    if (dtype == 0) SAMPLE_SIZES(__nv_bfloat16);
-    else SAMPLE_SIZES(float);
-#undef SAMPLE_SIZES
-#undef SAMPLE_LAUNCH
-    return 0;
+  const bool cluster = V >= 4096 && V <= 8 * SAMPLE_CT * 64 && sample_cluster_enabled();
+  // CTAs a row: as many as leave one for every SM (half of them in clusters of eight, which want eight SMs of a GPC), and so
+  // many that a thread has at most 32 keys (then two fit an SM); a barrier over a larger cluster costs more than the
+  // shorter passes give.  200 rows of 32000, p = 0.95: 258 us with eight, 147 with four, 138 with two, 170 with one; 32
+  // rows: 44, 38, 61, 88; 16 rows of 8192: 37, 28, 30, 36; 8 rows of 50000: 40, 59, 85.
+  int cl = 8;
+  while (cl > 1 && R * cl > (cl == 8 ? 74 : 148) && V <= cl / 2 * SAMPLE_CT * 32) cl /= 2;
+  // Rows of which nothing is cut take one pass: with many long rows the single-CTA kernel, which has more threads on an SM,
+  // is the faster one for them, and the cluster kernel leaves them out (an empty launch, 6 us, for the others).  Per round of
+  // clusters (two CTAs an SM up to 32 keys a thread, else one) 33 or 27 us; V / 1140 us for 148 rows of a CTA.  148 rows of
+  // 151936: 127 us there, 205 in clusters; 64 rows: 127 and 102.
+  const bool two = V <= cl * SAMPLE_CT * 32;
+  const int split = cluster && cl >= 4 &&
+                    (two ? 33.f / 296 : 27.f / 148) * R * cl > (R > 148 ? 1.7f : 1.f) * (float)V / 1140.f + 6.f;
+  if (!cluster || split) {
+    if (dtype == 0)
+      sample_kernel<__nv_bfloat16><<<R, SAMPLE_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, ld, V, temperature, top_k,
+                                                                    top_p, uniform, seed, step, step_ptr, out, split);
+    else
+      sample_kernel<float><<<R, SAMPLE_THREADS, 0, stream>>>((const float*)logits, ld, V, temperature, top_k, top_p, uniform,
+                                                            seed, step, step_ptr, out, split);
+    B200_CUDA_CHECK(cudaGetLastError());
+    if (!cluster) return 0;
   }
-  if (dtype == 0)
-    sample_kernel<__nv_bfloat16><<<R, SAMPLE_THREADS, 0, stream>>>((const __nv_bfloat16*)logits, ld, V,
-                                                                  temperature, top_k, top_p, uniform, seed,
-                                                                  step, step_ptr, out);
-  else
-    sample_kernel<float><<<R, SAMPLE_THREADS, 0, stream>>>((const float*)logits, ld, V, temperature, top_k,
-                                                          top_p, uniform, seed, step, step_ptr, out);
-  B200_CUDA_CHECK(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(R * cl);
+  cfg.blockDim = dim3(SAMPLE_CT);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  // the smallest instance that holds the row: passes run over all keys of a thread
+#define SAMPLE_LAUNCH(T, NPT, CL)                                                                                          \
+  B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, sample_cluster_kernel<T, NPT, CL>, (const T*)logits, ld, V, temperature, top_k, \
+                                     top_p, uniform, seed, step, step_ptr, out, split))
+#define SAMPLE_SMALL(T, CL)                                       \
+  do {                                                            \
+    if (V <= CL * SAMPLE_CT * 8) SAMPLE_LAUNCH(T, 8, CL);         \
+    else if (V <= CL * SAMPLE_CT * 16) SAMPLE_LAUNCH(T, 16, CL);  \
+    else SAMPLE_LAUNCH(T, 32, CL);                                \
+  } while (0)
+#define SAMPLE_SIZES(T)                                           \
+  do {                                                            \
+    if (cl == 1) SAMPLE_SMALL(T, 1);                              \
+    else if (cl == 2) SAMPLE_SMALL(T, 2);                         \
+    else if (cl == 4) SAMPLE_SMALL(T, 4);                         \
+    else if (V <= 8 * SAMPLE_CT * 32) SAMPLE_SMALL(T, 8);         \
+    else if (V <= 8 * SAMPLE_CT * 40) SAMPLE_LAUNCH(T, 40, 8);    \
+    else SAMPLE_LAUNCH(T, 64, 8);                                 \
+  } while (0)
+  if (dtype == 0) SAMPLE_SIZES(__nv_bfloat16);
+  else SAMPLE_SIZES(float);
+#undef SAMPLE_SIZES
+#undef SAMPLE_SMALL
+#undef SAMPLE_LAUNCH
   return 0;
 }
 
