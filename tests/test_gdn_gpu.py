@@ -212,3 +212,20 @@ def test_states_at_any_address(q_lens, ctx, off):
         # fp32 sums of 128 products in another order (2^-24 * sqrt(128) * a few), bf16 outputs
         torch.testing.assert_close(apart, want_rec, rtol=1e-4, atol=1e-5)
         torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -7, atol=1e-4)
+
+
+def test_rows_of_a_step_without_requests_are_zeros():
+    from vllm_torchtpu_b200.ops import cuda
+    Hk, Hv, D, T = 1, 2, 128, 6
+    C = (2 * Hk + Hv) * D
+    meta = _meta([], [], [])
+    used = torch.full((T * C * 8,), float("nan"), device=DEV).bfloat16()
+    del used                                                 # (the next tensors lie there)
+    x, a = torch.ones(T, C, device=DEV).bfloat16(), torch.ones(T, Hv, device=DEV).bfloat16()
+    pools = torch.zeros(1, C, 3, device=DEV).bfloat16(), torch.zeros(1, Hv, D, D, device=DEV)
+    w, A, dt = torch.ones(C, 4, device=DEV).bfloat16(), torch.zeros(Hv, device=DEV), torch.zeros(Hv, device=DEV)
+    q, v = torch.ones(T, Hk, D, device=DEV).bfloat16(), torch.ones(T, Hv, D, device=DEV).bfloat16()
+    for y in (cuda.gdn_forward(x, a, a, meta, *pools, w, A, dt, Hk, Hv, D, D), cuda.short_conv(x, meta, pools[0], w),
+              cuda.kda_forward(q, q, v, torch.ones(T, Hv, D, device=DEV).bfloat16(), a, meta, pools[1], A,
+                               torch.zeros(Hv, D, device=DEV))):
+        assert y.eq(0).all()

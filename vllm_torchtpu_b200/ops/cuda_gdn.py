@@ -22,6 +22,11 @@ def chunk_scratch_bytes(max_tokens: int, max_reqs: int, Hv: int) -> int:
     return 4 * min(MOST_WORDS, chunk_words(max_tokens, max_reqs, Hv))
 
 
+def _rows(R: int, *shape, device):
+    """Output rows; the kernels write all of them, zeros where there is no request, unless there is none at all."""
+    return (torch.empty if R > 0 else torch.zeros)(shape, dtype=torch.bfloat16, device=device)
+
+
 def gdn_forward(mixed, a, b, meta, conv_pool, rec_pool, conv_w, A_log, dt_bias, Hk, Hv, dk, dv):
     """mixed [T, 2*Hk*dk + Hv*dv] bf16 (may be a column slice), a/b [T, Hv] -> o [T, Hv, dv]."""
     _c._require_bf16(mixed, a, b, conv_w)
@@ -30,7 +35,7 @@ def gdn_forward(mixed, a, b, meta, conv_pool, rec_pool, conv_w, A_log, dt_bias, 
     R = meta.padded_num_reqs if meta.padded_num_reqs is not None else meta.num_reqs
     def new(*shape, dtype=torch.float32):
         return torch.empty(shape, dtype=dtype, device=dev)
-    out = new(T, Hv, dv, dtype=torch.bfloat16)
+    out = _rows(R, T, Hv, dv, device=dev)
     conv_out = qn = kn = g = beta = chunks = None
     # single tokens have their own kernel, which reads weights in pieces of 8 bytes and states in pieces of 16
     step = dk == dv == 128 and conv_w.data_ptr() % 8 == 0 and rec_pool.data_ptr() % 16 == 0
@@ -70,7 +75,7 @@ def kda_forward(q, k, v, a, b, meta, rec_pool, A_log, dt_bias, lower_bound=None)
     kn = torch.empty_like(qn)
     g = torch.empty((T, Hv, dk), dtype=torch.float32, device=dev)
     beta = torch.empty((T, Hv), dtype=torch.float32, device=dev)
-    out = torch.empty((T, Hv, dv), dtype=torch.bfloat16, device=dev)
+    out = _rows(R, T, Hv, dv, device=dev)
     A_log = A_log.float().contiguous()
     dt_bias = dt_bias.float().contiguous()
     lb = float(lower_bound) if lower_bound is not None else 0.0
@@ -89,7 +94,7 @@ def short_conv(x, meta, conv_pool, conv_w):
     _c._require_bf16(x, conv_w)
     T, C = x.shape
     R = meta.padded_num_reqs if meta.padded_num_reqs is not None else meta.num_reqs
-    y = torch.empty((T, C), dtype=torch.bfloat16, device=x.device)
+    y = _rows(R, T, C, device=x.device)
     _c._check(_c.lib().b200_short_conv(
         _c._p(x), c_int(x.stride(0)), _c._p(conv_w), _c._p(conv_pool), _c._p(y), _c._p(meta.query_start_loc),
         _c._p(meta.seq_lens), _c._p(meta.state_slots), c_int(R), c_int(T), c_int(C), c_int(conv_w.shape[1]), _c._stream()),
