@@ -229,3 +229,36 @@ def test_rows_of_a_step_without_requests_are_zeros():
               cuda.kda_forward(q, q, v, torch.ones(T, Hv, D, device=DEV).bfloat16(), a, meta, pools[1], A,
                                torch.zeros(Hv, D, device=DEV))):
         assert y.eq(0).all()
+
+
+def test_chunks_keep_32_bits():
+    """Chunks against the rule in 64 bits on the kernel's own convolved rows: 24 chunks with slow decay.  States and sums are
+    fp32, every fp32 operand enters as three parts: a lost part would show as 2^-9 or 2^-17."""
+    from vllm_torchtpu_b200.ops import cuda
+    gen = torch.Generator(device=DEV).manual_seed(13)
+    Hk, Hv, D, T = 1, 2, 128, 24 * 64 + 9
+    C = (2 * Hk + Hv) * D
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)                      # noqa: E731
+    mixed, a, b = rnd(T, C).bfloat16(), (rnd(T, Hv) * 0.3 - 7).bfloat16(), rnd(T, Hv).bfloat16()
+    conv_w, A_log, dt = (rnd(C, 4) * 0.3).bfloat16(), rnd(Hv) * 0.3, rnd(Hv) * 0.3
+    meta = _meta([T], [64], [0])
+    conv, rec = rnd(1, C, 3).bfloat16(), rnd(1, Hv, D, D) * 0.1
+    y = cuda.short_conv(mixed, meta, conv.clone(), conv_w).double()
+    got_rec = rec.clone()
+    got = cuda.gdn_forward(mixed, a, b, meta, conv.clone(), got_rec, conv_w, A_log, dt, Hk, Hv, D, D)
+    q, k, v = (t.reshape(T, -1, D) for t in y.split([Hk * D, Hk * D, Hv * D], -1))
+    q, k = (torch.nn.functional.normalize(t, dim=-1).repeat_interleave(Hv // Hk, 1) for t in (q, k))
+    decay = torch.exp(-A_log.double().exp() * torch.nn.functional.softplus(a.double() + dt.double()))
+    S, beta = rec[0].double(), b.double().sigmoid()
+    want = torch.empty(T, Hv, D, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        S = S * decay[t][:, None, None]
+        u = (v[t] - torch.einsum("hk,hkv->hv", k[t], S)) * beta[t][:, None]
+        S = S + k[t][:, :, None] * u[:, None]
+        want[t] = torch.einsum("hk,hkv->hv", q[t], S) * D ** -0.5
+
+    def rel(x, y):
+        return float((x.double() - y).norm() / y.norm())
+    # decays from the fast exponential and logarithm (2^-21 a token, a memory of some hundred tokens): about 1e-6
+    assert rel(got_rec[0], S) < 1e-5
+    assert rel(got, want) < 2.5e-3                           # bf16 outputs: 2^-9 at most, 2^-9 / sqrt(3) in the norm

@@ -70,6 +70,43 @@ def test_mla_tiles_of_128_rows(q_lens, ctx, H):
     _case(q_lens, ctx, H, 512, 64)
 
 
+# pages of more than 16 rows: several copies of a page, pages that end inside a chunk of 128 keys
+@pytest.mark.parametrize("bs", [32, 48, 64, 128])
+def test_mla_pages_of_more_rows(bs):
+    _case([1, 1, 1, 70, 5], [0, bs - 1, bs, 430, 131], 16, 512, 64, bs=bs)
+    _case([1] * 3, [1000, 129, 2050], 128, 512, 64, bs=bs)
+
+
+def test_mla_captured_step_with_more_splits_than_chunks():
+    """The splits of a captured step follow from the batch; replayed on short contexts most of them see no key."""
+    from vllm_torchtpu_b200.ops import cuda
+    g = torch.Generator(device=DEV).manual_seed(4)
+    R, H, L = 4, 16, 512
+    cache = torch.randn(1 + R * 64, 16, 576, device=DEV, generator=g).bfloat16()
+    bt = (torch.randperm(R * 64, device=DEV, generator=g) + 1).to(torch.int32).view(R, 64).contiguous()
+    q = torch.randn(R, H, 576, device=DEV, generator=g).bfloat16()
+    sl = torch.full((R,), 1000, dtype=torch.int32, device=DEV)
+    qsl = torch.arange(R + 1, dtype=torch.int32, device=DEV)
+    meta = AttentionMetadata(None, None, bt, sl, qsl, R, R, num_decode_reqs=R, max_query_len=1, max_seq_len=1000,
+                             padded_num_reqs=R, padded_num_tokens=R)
+    cuda.mla_paged_attention(q, cache, meta, 576 ** -0.5, L)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = cuda.mla_paged_attention(q, cache, meta, 576 ** -0.5, L)
+    for lens in ([1, 16, 129, 300], [1024, 3, 640, 128], [0, 1, 0, 5]):
+        sl.copy_(torch.tensor(lens, dtype=torch.int32))
+        graph.replay()
+        for r, n in enumerate(lens):
+            if n == 0:
+                assert out[r].eq(0).all()
+                continue
+            rows = cache[bt[r].long()].view(-1, 576)[:n].double()
+            want = torch.softmax(q[r].double() @ rows.t() * 576 ** -0.5, -1) @ rows[:, :L]
+            assert (out[r].double() - want).norm() / want.norm() < 2 ** -7
+    assert cuda.check_status() == 0
+
+
 def test_mla_rows_of_the_cache_that_nothing_wrote_do_not_matter():
     from vllm_torchtpu_b200.ops import cuda
     g = torch.Generator(device=DEV).manual_seed(3)
