@@ -17,11 +17,13 @@
 //               exact weight 1 of the largest score: 0.0020 instead of 0.0018 from the result in 64 bits.)
 // Query rows 73.7 KB, K 73.7 KB, V 65.5 KB, P 16.4 KB of shared memory: single buffers, refilled by parts (K in three
 // groups of panels, V in two halves) while the other product runs, which leaves a part about 1700 cycles to arrive.
-// Persistent: pairs take (tile, split) items, the longest first.  Two warps copy, one issues, eight compute.
+// Persistent: pairs take (tile, split) items from the last request to the first and, in a request, from its last tokens,
+// which see the most keys, to its first.  (Decoding requests stand first in a batch: they come last, whatever their length.)
+// Two warps copy, one issues, eight compute.
 //
-// Measured on B200 (CUDA events), 128 heads, mma.sync kernel -> this one: 4 x 2048 prompt tokens 32.5 -> 2.23 ms (71.9 -> 1050
-// TFLOP/s), 64 requests of 0.9 to 2 K keys 567 -> 61 us.  A chunk takes about 4500 cycles where its products need 2176:
-// K and V arrive late.  What mattered on the way: one elected thread issues (44 -> 32 cycles per product of N = 128),
+// Measured on B200 (CUDA events), 128 heads, mma.sync kernel -> this one: 4 x 2048 prompt tokens 32.5 -> 2.22 ms in short runs, 2.58 in
+// long ones under the power cap (71.9 -> 1050 and 905 TFLOP/s), 64 requests of 0.9 to 2 K keys 567 -> 61 us.  A chunk takes about
+// 4500 cycles where its products need 2176.  What mattered on the way: one elected thread issues (44 -> 32 cycles per product of N = 128),
 // the one arrival a chunk on the leader's barrier releases shared memory at cluster scope (all memory: 2.22 -> 2.73 ms),
 // K and V have a copying warp each with the table entries fetched ahead.
 //

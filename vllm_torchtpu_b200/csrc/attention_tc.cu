@@ -11,12 +11,14 @@
 //                    contiguous), result in TMEM (two buffers); the softmax threads fold it into
 //                    their fp32 register accumulators (acc = acc * alpha + O_chunk), so TMEM is
 //                    never rescaled in place.
-// Warp roles: warp 0 TMA producer (Q tile once, K and V rings, one 16-token page per copy), warp 1
-// MMA issuer, warps 2-9 softmax + output (two threads per row, one per half of the key columns).  S(j+1) is issued before P V(j), so the tensor core works
-// on the next scores while the softmax of the current chunk runs.  512 TMEM columns, 226 KB of
-// shared memory.  What bounds it: the chain scores -> softmax -> P V of a chunk; the tensor work of a chunk is 1024 cycles.
+// Warp roles: warp 0 TMA producer (Q of this tile and the next, K and V rings, one page of 16 tokens per lane and copy), warp 1
+// MMA issuer, warps 2-9 softmax + output (two threads per row, one per half of the key columns).  S(j+1) is issued before
+// P V(j), so the tensor core works on the next scores while the softmax of the current chunk runs.  512 TMEM columns, 226 KB
+// of shared memory.  What bounds it: the chain scores -> softmax -> P V of a chunk; the tensor work of a chunk is 1024 cycles.
 // 8 x 1024 tokens, 32 / 8 heads: 237 us with a CTA per tile, the scores read twice from TMEM and K, V and the table entry
-// waited for together; 223 us persistent with the scores read once; 196 to 203 us with K and V copied as their buffers come free.  Every mbarrier wait is bounded (status word + abort flag + TMEM freed on exit).
+// waited for together; 223 us persistent with the scores read once; 200 us with K and V copied as their buffers come free;
+// 185 us with capped scores in an instance of their own (fewer registers in this one), 181 us with rounds of tiles back and
+// forth.  Every mbarrier wait is bounded (status word + abort flag + TMEM freed on exit).
 //
 // Same function as the mma.sync prefill kernel in attention.cu (causal ragged batches with prefix
 // context, sliding window, soft-cap, sinks, LSE); semantics of the reference's ragged paged
@@ -30,7 +32,7 @@ namespace b200 {
 namespace fa {
 
 constexpr int D = 128;
-constexpr int BM = 128;                  // query rows per CTA
+constexpr int BM = 128;                  // query rows per tile
 constexpr int BKV = 128;                 // keys per chunk
 constexpr int HALF_BYTES = 128 * 128;    // 128 rows x 64 bf16: one swizzled half of a 128 x 128 tile
 constexpr int TILE_BYTES = 2 * HALF_BYTES;

@@ -1,10 +1,11 @@
 // Gated DeltaNet kernels: causal depth-wise conv1d with a carried window, gate/normalisation
 // prep, and the gated delta-rule recurrence with the per-head state held in registers.
 //
-// The recurrence runs one CTA per (request, value head, 64 columns of the [dk, dv] state); columns are independent
-// of each other.  The same kernel serves decode (one token) and prefill (the request's tokens in order);
-// parallelism comes from requests x heads x columns.  State lives in pools indexed by
-// the request's slot; a request whose first token of the step has position 0 starts from zero.
+// Heads of 128 / 128: single tokens take delta_step_kernel (everything in one launch), longer portions of the scalar rule
+// the chunks of gdn_chunk.cu.  Other portions, head sizes and the channel rule take the recurrence: one CTA per
+// (request, value head, 64 columns of the [dk, dv] state), the request's tokens in order; columns are independent of each
+// other.  State lives in pools indexed by the request's slot; a request whose first token of the step has position 0
+// starts from zero.
 //
 // Math of the reference's fused conv1d + GDN kernels (reference: src/vllm_torchtpu/kernels/gdn/v3/),
 // which use a chunked WY form for prefill; the recurrence below is the same function.
@@ -41,8 +42,9 @@ struct Row<8> {
 // to 32 tokens of one request and 128 * VEC channels, with the three tokens in front of them.  Bound by memory: one read
 // and one write of the rows; eight rows of a thread are in flight.  Only the CTA of a request's first tokens touches
 // the carried window: it reads the old one and writes the new one.  Rows of no request become zeros.
-// 4 x 2048 tokens and 8192 channels take 100 us (2.7 TB/s): the exponential
-// and the reciprocal of every value.  One thread per channel through all tokens of a request had one load in flight.
+// 4 x 2048 tokens and 8192 channels take 100 us (2.7 TB/s): the next eight rows are loaded only once the present ones are
+// stored, and every CTA begins with a search, its weights and a halo.  (The division is IEEE's: 3 us of the 100.)  One
+// thread per channel through all tokens of a request had one load in flight.
 template <int VEC>
 __global__ void __launch_bounds__(128)
 gdn_conv_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, __nv_bfloat16* conv_pool,

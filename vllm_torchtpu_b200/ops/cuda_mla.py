@@ -29,7 +29,8 @@ def _mla_tc(q, cache, meta, scale, R, return_lse):
     ws = _c.Workspace.get(q.device)
     out = torch.empty((T, H, 512), dtype=q.dtype, device=q.device)
     lse = torch.empty((T, H), dtype=torch.float32, device=q.device) if return_lse else None
-    # split-KV when the tiles of 128 rows are fewer than the pairs of SMs.  Inside a captured graph the choice depends on the
+    # split-KV when the tiles of 128 rows are at most half as many as the SMs (a tile takes a pair of them: up to two rounds of
+    # items), in at most 16 parts of 128 keys or more.  Inside a captured graph the choice depends on the
     # batch shape only (lengths change between replays; a split without keys contributes lse = -inf).
     tiles = max(R, T * H // 128)
     splits = max(1, min(16, _c._sms // max(1, tiles)))
